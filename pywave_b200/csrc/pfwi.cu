@@ -5,12 +5,10 @@
 // Scheme (pywave/src/wave_fwimodeling.c:72-104, wave_fwigradient.c:132-241):
 //   term = Lap8(a) (zero outside [4,pad-4)) + rr*w[it]
 //   a_new = S((2a - S(b)) + (v*v*dt^2)*term),   S = sponge, b = previous a
-// on the padded grid (nz+2nb) x (nx+2nb).  Same field layout, two-buffer
-// scheme and cp.async plane pipeline as the afd kernel, with an 8th-order
-// stencil: the model's x is the marched axis (9-deep register queue), z is
-// tiled (float4 per thread, one float4 of halo on each side = 4 cells).
-// All shots of a call advance together, one after another inside each CTA,
-// sharing the v^2 dt^2 plane.
+// on the padded grid (nz+2nb) x (nx+2nb).  Field layout and two-buffer scheme
+// of the afd kernels, with an 8th-order stencil; a thread updates one float4
+// of z cells of one x plane.  All shots of a batch advance together in one
+// launch per step, sharing V = v^2 dt^2.
 #include "pw_common.cuh"
 
 #include <algorithm>
@@ -24,6 +22,7 @@ namespace pf {
 
 constexpr int HZ = 4;        // z halo (cells) in front of iz = 0
 constexpr int HX = 4;        // x halo (planes) in front of ix = 0
+constexpr int PF_XW = 4;     // x planes (warps) per CTA of the step kernel
 constexpr int MAXS = 64;     // shots per launch
 constexpr int MAXSRCW = 16;  // source-map cells per shot
 
@@ -46,32 +45,27 @@ enum Mode { FWD = 0, ADJ_REF = 1, ADJ_EXACT = 2 };
 // divisor is checked on the GPU against __fdiv_rn for all 2^23 significands
 // of x in one binade; scaling x by 2^k scales every step exactly while the
 // intermediate values stay normal, which |x| in [xmin, xmax] ensures.
-// Below xmin (the tiny values at the edge of a wavefield, subnormal ones
-// included) div_small scales x by 2^89 into that range, divides, and scales
-// back, which is exact unless the quotient is subnormal and the scaled
-// quotient sits exactly on a tie of the subnormal grid; there the sign of
-// the exact remainder xs - qs*d (one FMA) picks the side.  The setup checks
-// it against __fdiv_rn for every float in (0, xmin) as well.
-// Above xmax, for NaN or infinity, or when a check fails: __fdiv_rn.
+// Below xmin (the tiny values at the edge of a wavefield) and above xmax, or
+// when the check fails: div_f64; for NaN or infinity: __fdiv_rn.
 struct DivC {
-  float d, zh, zl, xmin, xmax;
-  int ok;
-  unsigned int umin, uspan, umax;  // bits of xmin; of xmax minus xmin; of xmax
-  float sup, sdn, sgrid;           // 2^K, 2^-K, 2^(149-K) for div_small
+  float d, zh, zl, xmin, xmax;  // xmin > xmax: no numerator takes the method
+  double dd, rd;                // d and RN(1/d)
 };
-constexpr int DIV_SMALL_K = 89;
 
 struct PfArgs {
   int pnz, pnx;               // padded grid
   int lz;                     // leading dimension of the field layout
   int nb, nz, nx;             // sponge width, interior
   float c0, c1, c2, c3, c4;   // 8th-order coefficients (wave_fwiutil.c:17)
-  float dx2, dz2;
   float one;                  // 1.0f at run time: keeps packed products unfused (pk2 helpers)
   DivC divx, divz;            // fast exact division by dx2 / dz2
-  int nshots;
-  const float *cur[MAXS];
-  float *nxt[MAXS];
+  float xlo, xhi;             // numerators that both divide as they are
+  int nz4;                    // float4 per padded column
+  unsigned div_m, div_s;      // n / nz4 = umulhi(n, div_m) >> div_s for n < 2^31
+  int src_z0, src_z1;         // rows of the shots' source cells
+  const float *cur;           // the shots' current fields, fstep floats apart
+  float *nxt;                 // the shots' previous fields, overwritten with the next
+  long long fstep;
   const float *V;             // v*v*dt^2 (field layout)
   const float *bz, *bx;       // sponge factor per z / x cell (1 off the faces)
   int it, nt;
@@ -96,8 +90,7 @@ struct PfArgs {
   long long gstride;          // floats between the shots' gradient slices (0: one accumulator)
   const float *tin;           // ADJ_EXACT: term of the forward step [shot] (field layout)
   long long tin_stride;
-  int imaging;                // this step images
-  long long fstride;          // field size (floats)
+  int imaging;                // ADJ_REF: this step images
 };
 
 __device__ __forceinline__ float el(const float4 &v, int e) {
@@ -116,376 +109,291 @@ __device__ __forceinline__ void cp16(float4 *dst, const float *src, bool valid) 
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(src), "r"(n)
                : "memory");
 }
-__device__ __forceinline__ void cp4(float *dst, const float *src, bool valid) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(dst);
-  const int n = valid ? 4 : 0;
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(s), "l"(src), "r"(n)
-               : "memory");
-}
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// z terms of the 8th-order Laplacian for cell e of the float4 c, with L / R
-// the float4s below and above (cells -4..-1, +4..+7).
-__device__ __forceinline__ float znb(const float4 &L, const float4 &c, const float4 &R, int e, int d) {
-  const int j = e + d;  // -4 .. 7
-  if (j < 0) return el(L, j + 4);
-  if (j > 3) return el(R, j - 4);
-  return el(c, j);
+// largest / smallest |x| of three (a NaN wins the maximum)
+__device__ __forceinline__ float max3abs(float a, float b, float c) {
+  float r;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float min3abs(float a, float b, float c) {
+  float r;
+  asm("min.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
 }
 
-__device__ __forceinline__ float div_bmr(float x, const DivC &c) {
-  // copysignf keeps the sign of a zero quotient (d > 0)
-  return copysignf(__fmaf_rn(x, c.zh, __fmul_rn(x, c.zl)), x);
+// v / d rounded once, through FP64: q = v * RN(1/d) corrected by its exact
+// remainder is v / d to within a rounding of 53 bits, and equals it where
+// v / d has at most 53 bits; a quotient of two floats that is no tie of the
+// float grid (subnormal or not) lies at least 2^-48 of itself from every
+// tie, so rounding q to float gives the correctly rounded quotient.
+__device__ __forceinline__ float div_f64(float v, double d, double rd) {
+  const double x = (double)v, q = __dmul_rn(x, rd);
+  return __double2float_rn(__fma_rn(__fma_rn(-q, d, x), rd, q));
 }
 
-__device__ __forceinline__ float div_small(float x, const DivC &c) {
-  const float xs = __fmul_rn(x, c.sup);  // exact, inside [xmin, xmax]
-  const float qs = __fmaf_rn(xs, c.zh, __fmul_rn(xs, c.zl));
-  const float q = copysignf(__fmul_rn(qs, c.sdn), x);
-  const float t = fabsf(__fmul_rn(qs, c.sgrid));  // |qs| in units of 2^-149 (exact)
-  const float n = truncf(t);
-  if (t - n == 0.5f) {
-    const float r = __fmaf_rn(-qs, c.d, xs);  // exact remainder
-    if (r != 0.f)
-      return __uint_as_float((__float2uint_rz(n) + ((r > 0.f) == (x > 0.f) ? 1u : 0u)) |
-                             (__float_as_uint(x) & 0x80000000u));
-  }
-  return q;
-}
-
-// div_bmr on a pair: the same fused product and the sign of x per lane
-__device__ __forceinline__ f2 div_bmr2(f2 x, f2 zh, f2 zl) {
-  const f2 q = fma2(x, zh, mul2(x, zl));
-  return (q & 0x7fffffff7fffffffull) | (x & 0x8000000080000000ull);
-}
-
-// tx[e]/cx.d and tz[e]/cz.d for the 4 cells of a float4, correctly rounded.
-// The lanes of `mask` vote once: every numerator zero or in [xmin, xmax]
-// runs div_bmr (two values per op); every one below xmax runs div_small or
-// div_bmr per value; otherwise __fdiv_rn (a per-value choice of all three
-// would be if-converted into every sequence).  Any grouping of lanes is
-// correct, as every lane's own vote is in its group.
-__device__ __forceinline__ void div4x2(const float (&tx)[4], const float (&tz)[4],
-                                       const DivC &cx, const DivC &cz, unsigned mask,
-                                       float (&qx)[4], float (&qz)[4]) {
-  // |x| in [xmin, xmax] or 0 for all four: the largest |x| bits at most
-  // umax, and the smallest of |x| bits - 1 (a zero wraps to the top and
-  // drops out) at least umin - 1; positive floats order as their bits
-  unsigned mxx = 0u, mxz = 0u, mnx = ~0u, mnz = ~0u;
+// tx / cx.d + tz / cz.d for the two pairs of cells of a float4, each quotient
+// correctly rounded.  Every |numerator| in [xlo, xhi], the common part of the
+// divisors' [xmin, xmax], or no result used (`unused`): the constant-divisor
+// method, two values per op.  All zero (ahead of the numerical wavefront):
+// zero.  Otherwise (the shell of tiny values around that zone, which crosses
+// most columns while a wave expands) through FP64, or by __fdiv_rn where a
+// numerator is infinite or NaN.  The first test is 8 three-operand minima and
+// maxima for the 8 numerators.
+// The sign of a zero quotient is not kept (these forms can give +0 for -0):
+// no output depends on it.  The sum of the quotients is then +0 where it
+// should be -0 only if both numerators are -0, for which the centre value c
+// must be +0 (c0 c is +0 for c = -0, and a sum that starts at +0 never
+// becomes -0); the update (2c - b) + V t has 2c - b = +0 - b, which is not
+// -0, so adding +0 or -0 gives the same bits, and the gradient sums start at
+// +0, which adding either zero leaves unchanged.
+__device__ __forceinline__ void div4_sum(const f2 (&tx)[2], const f2 (&tz)[2], const DivC &cx,
+                                         const DivC &cz, float xlo, float xhi, bool unused,
+                                         f2 (&t)[2]) {
+  const float4 x = join2(tx[0], tx[1]), z = join2(tz[0], tz[1]);
+  const float mx = max3abs(max3abs(max3abs(x.x, x.y, x.z), x.w, z.x), z.y, max3abs(z.z, z.w, 0.f));
+  const float mn = min3abs(min3abs(min3abs(x.x, x.y, x.z), x.w, z.x), z.y, min3abs(z.z, z.w, z.w));
+  const f2 xh = pk2(cx.zh, cx.zh), xl = pk2(cx.zl, cx.zl);
+  const f2 zh = pk2(cz.zh, cz.zh), zl = pk2(cz.zl, cz.zl);
+  if (unused || (mn >= xlo && mx <= xhi)) {
 #pragma unroll
-  for (int e = 0; e < 4; e++) {
-    const unsigned ux = __float_as_uint(tx[e]) & 0x7fffffffu;
-    const unsigned uz = __float_as_uint(tz[e]) & 0x7fffffffu;
-    mxx = max(mxx, ux);
-    mxz = max(mxz, uz);
-    mnx = min(mnx, ux - 1u);
-    mnz = min(mnz, uz - 1u);
+    for (int h = 0; h < 2; h++)
+      t[h] = add2(fma2(tx[h], xh, mul2(tx[h], xl)), fma2(tz[h], zh, mul2(tz[h], zl)));
+    return;
   }
-  const bool ok = cx.ok && cz.ok;
-  const bool in = ok && mxx <= cx.umax && mxz <= cz.umax && mnx >= cx.umin - 1u &&
-                  mnz >= cz.umin - 1u;
-  if (__all_sync(mask, in)) {
-    const f2 xh = pk2(cx.zh, cx.zh), xl = pk2(cx.zl, cx.zl);
-    const f2 zh = pk2(cz.zh, cz.zh), zl = pk2(cz.zl, cz.zl);
-    up2(div_bmr2(pk2(tx[0], tx[1]), xh, xl), qx[0], qx[1]);
-    up2(div_bmr2(pk2(tx[2], tx[3]), xh, xl), qx[2], qx[3]);
-    up2(div_bmr2(pk2(tz[0], tz[1]), zh, zl), qz[0], qz[1]);
-    up2(div_bmr2(pk2(tz[2], tz[3]), zh, zl), qz[2], qz[3]);
-  } else if (__all_sync(mask, ok && mxx <= cx.umax && mxz <= cz.umax)) {
+  t[0] = t[1] = 0ull;
+  if (mx == 0.f) return;
+  float4 r;
+  if (mx <= FLT_MAX) {
 #pragma unroll
-    for (int e = 0; e < 4; e++) {
-      const bool sx = (__float_as_uint(tx[e]) & 0x7fffffffu) < cx.umin;
-      const bool sz = (__float_as_uint(tz[e]) & 0x7fffffffu) < cz.umin;
-      qx[e] = sx ? div_small(tx[e], cx) : div_bmr(tx[e], cx);
-      qz[e] = sz ? div_small(tz[e], cz) : div_bmr(tz[e], cz);
-    }
+    for (int e = 0; e < 4; e++)
+      set_el(r, e, fadd(div_f64(el(x, e), cx.dd, cx.rd), div_f64(el(z, e), cz.dd, cz.rd)));
   } else {
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-      qx[e] = __fdiv_rn(tx[e], cx.d);
-      qz[e] = __fdiv_rn(tz[e], cz.d);
-    }
+#pragma unroll 1
+    for (int e = 0; e < 4; e++) set_el(r, e, fadd(__fdiv_rn(el(x, e), cx.d), __fdiv_rn(el(z, e), cz.d)));
   }
+  t[0] = lo2(r);
+  t[1] = hi2(r);
 }
 
-// One pfwi step over a z column segment of ZW float4 marching along x.
-template <int ZW, int P, int MODE, bool PAS = false>
-__global__ void __launch_bounds__(ZW) pf_step_kernel(const PfArgs a, int xch) {
-  constexpr int W = ZW + 2;   // curr plane (float4) incl. z halo
-  constexpr int NC = P + 10;  // curr planes (x-4..x+4 live, P ahead, 1 slack)
-  constexpr int NP = P + 2;
-  extern __shared__ float4 sm[];
-  float4 *s_cur = sm;
-  float4 *s_prev = sm + NC * W;
-  float4 *s_V = s_prev + NP * ZW;
-  float4 *s_t = s_V + NP * ZW;  // ADJ_EXACT: forward term tile
-  float4 *s_g = s_t + NP * ZW;  // ADJ_EXACT: this shot's gradient slice
-  float4 *s_d = s_t;            // FWD with passive sources: the step's source field
+__device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 
-  const int tid = threadIdx.x;
-  const int s = blockIdx.x;  // shot of the batch: fastest, so the shots of one x chunk
-                             // run together and share V through L2
-  const int z4 = blockIdx.z * ZW + tid;
+// One pfwi step: a thread updates one float4 of z cells (z4) of one x plane of
+// one shot, straight from global memory (9 loads of its own column, the two z
+// neighbours, the previous field and V; for the adjoint the forward term and
+// the gradient).  No march, no shared memory, no barrier: the registers of
+// one plane (80) leave 24 warps per SM to hide the load latency.  Lanes are
+// numbered z4 + nz4 * (group of PF_XW planes) without regard to columns, so
+// none is idle whatever the padded depth; the PF_XW warps of a CTA take the
+// planes of the group, whose 9-plane columns overlap in L1.
+// Bound: instruction issue and L1 / L2 latency (a 16-shot field pair of 420 x
+// 720 sits in L2).  Measured, one launch: 16 shots of 420 x 720, forward and
+// exact adjoint together 20.2 us on average (39.5 with the former x march of
+// 8 planes over a shared-memory ring: 626 instructions per float4, now 290);
+// 8 shots of 271 x 421 forward 6.4 us (16.1).  Marching 4 to 16 planes with
+// the 9-deep queue in registers ran 23 to 28 us, two planes per thread 20.7,
+// 8 planes per CTA 21.9, CTAs of consecutive lanes only 21.4.
+template <int MODE, bool PAS>
+__global__ void __launch_bounds__(32 * PF_XW, MODE == ADJ_REF || PAS ? 5 : 6)
+    pf_step_kernel(const __grid_constant__ PfArgs a) {
+  const int s = blockIdx.y;
+  const unsigned item = blockIdx.x * 32 + (threadIdx.x & 31);
+  const int chunk = (int)(__umulhi(item, a.div_m) >> a.div_s);  // item / nz4
+  const int z4 = (int)item - chunk * a.nz4;
+  const int x = chunk * PF_XW + (threadIdx.x >> 5);
   const int iz0 = 4 * z4;
-  const int x0 = blockIdx.y * xch;
-  const int x1 = min(a.pnx, x0 + xch);
-  const int nplanes = x1 - x0;
-  const int lz = a.lz;
-  const bool live = iz0 < a.pnz;
-  const long long o_c = pfoff(lz, iz0, 0);
-  const int ci = tid + 1;
-  const int hz4 = tid == 0 ? blockIdx.z * ZW - 1 : blockIdx.z * ZW + ZW;  // halo float4 (threads 0, 1)
-  const bool has_h = tid < 2;
-  const int hslot = tid == 0 ? 0 : ZW + 1;
-  const bool h_ok = has_h && hz4 >= -1 && hz4 * 4 < a.pnz;
-  const long long h_off = h_ok ? pfoff(lz, hz4 * 4, 0) : 0;
+  pdl_wait();
+  pdl_launch();
+  if (x >= a.pnx) return;
+  const long long lz = a.lz;
+  const long long o0 = pfoff(a.lz, iz0, x);  // own float4
+  const float *pc = a.cur + s * a.fstep + o0;
+  float *pn = a.nxt + s * a.fstep + o0;
+  const float *pv = a.V + o0;
+  const float *pt = MODE == ADJ_EXACT ? a.tin + s * a.tin_stride + o0 : nullptr;
+  float *pg = MODE == ADJ_EXACT ? a.grad + s * a.gstride + o0 : nullptr;
+  float *po = (MODE == FWD && a.tout) ? a.tout + s * a.tout_stride + o0 : nullptr;
+  float *const gs = MODE == ADJ_REF ? a.grad + s * a.gstride : nullptr;
 
-  float bzf[4];
-  bool lz_ok[4], zin[4];
+  float4 q[9];  // own column, planes x-4 .. x+4
 #pragma unroll
-  for (int e = 0; e < 4; e++) {
-    const int iz = iz0 + e;
-    bzf[e] = (live && iz < a.pnz) ? a.bz[iz] : 1.f;
-    lz_ok[e] = iz >= 4 && iz < a.pnz - 4;
-    zin[e] = iz < a.pnz;
+  for (int d = 0; d < 9; d++) q[d] = ld4(pc + (d - 4) * lz);
+  const float4 c = q[4], L = ld4(pc - 4), R = ld4(pc + 4), p4 = ld4(pn), V4 = ld4(pv);
+  float4 tf = make_float4(0.f, 0.f, 0.f, 0.f), g4 = tf;
+  if (MODE == ADJ_EXACT) {
+    tf = __ldcs(reinterpret_cast<const float4 *>(pt));
+    g4 = ld4(pg);
   }
+  const float bxf = a.bx[x];
+  const float4 bz4 = ld4(a.bz + iz0);
+  // the stencil's rows [4, pnz - 4): the first and the last float4 of a column
+  // hold none, at most one float4 holds some of both
+  const bool lz_any = z4 >= 1 && iz0 < a.pnz - 4;
+  const bool lz_full = lz_any && iz0 + 3 < a.pnz - 4;
   const bool rec_row = a.rz >= iz0 && a.rz < iz0 + 4;
+  const bool src_z = MODE == FWD && !PAS && iz0 <= a.src_z1 && iz0 + 3 >= a.src_z0;
+  const ShotGeo &sg = a.geo[s];
+  const f2 k1 = pk2(a.one, a.one);
+  const f2 kc[5] = {pk2(a.c0, a.c0), pk2(a.c1, a.c1), pk2(a.c2, a.c2), pk2(a.c3, a.c3),
+                    pk2(a.c4, a.c4)};
 
-  float *const gs = a.grad + s * a.gstride;  // this shot's gradient accumulator
+  // ADJ_REF imaging operands of this plane
+  double rw[4];
+  float rt[4], rg[4];
+  const bool xin = x >= a.nb && x < a.nb + a.nx;
+  const bool img = MODE == ADJ_REF && a.imaging && xin;
+  if (MODE == ADJ_REF) {
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      const int iz = iz0 + e;
+      rw[e] = 0.;
+      rt[e] = rg[e] = 0.f;
+      if (img && iz >= a.nb && iz < a.nb + a.nz) {
+        const size_t k = (size_t)(x - a.nb) * a.nz + (iz - a.nb);
+        const size_t ks = s * a.wstride + k;
+        // wave[wit+1] - 2.*wave[wit] + wave[wit-1] in double, left to right
+        rw[e] = __dadd_rn(__dsub_rn((double)a.wnext[ks], __dmul_rn(2., (double)a.wcur[ks])),
+                          (double)a.wprev[ks]);
+        rt[e] = a.m2v3[k];
+        rg[e] = gs[k];
+      }
+    }
+  }
+  float dv[4] = {0.f, 0.f, 0.f, 0.f};
+  if (MODE == FWD && PAS) {
+    // the interior cells' source samples
+    const float *row = a.dsrc + s * a.dsrc_stride +
+                       ((long long)a.it * a.nx + (xin ? x - a.nb : 0)) * a.nz;
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      const int iz = iz0 + e;
+      if (xin && iz >= a.nb && iz < a.nb + a.nz) dv[e] = __ldcs(row + (iz - a.nb));
+    }
+  }
+  // receivers read the field before the update (wave_fwimodeling.c:76-79)
+  int rir = -1;
+  if (rec_row) {
+    const int d = x - sg.r0v;
+    if (d >= 0) {
+      const int ir = a.drv == 1 ? d : (d % a.drv == 0 ? d / a.drv : -1);
+      if (ir >= 0 && ir < sg.nr2) rir = sg.r02 + ir;
+    }
+    if (MODE == FWD && rir >= 0 && a.rec)
+      a.rec[((size_t)s * a.nt + a.it) * a.nr + rir] = el(c, a.rz - iz0);
+  }
+  if (MODE == FWD && a.snap && xin) {
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      const int iz = iz0 + e;
+      if (iz >= a.nb && iz < a.nb + a.nz)
+        a.snap[s * a.snap_stride + (size_t)(x - a.nb) * a.nz + (iz - a.nb)] = el(c, e);
+    }
+  }
+  // the x and z sums of the 8th-order Laplacian in the reference's order,
+  // cells (0, 1) and (2, 3) of the float4 per f32x2 op; the z neighbours
+  // at odd distances are the float4s shifted by one cell
+  const f2 cl = lo2(c), ch = hi2(c);
+  const bool lx_ok = x >= 4 && x < a.pnx - 4;
+  f2 t2[2];
   {
-    const float *cur = a.cur[s];
-    float *nxt = a.nxt[s];
-    const float *tin = MODE == ADJ_EXACT ? a.tin + s * a.tin_stride : nullptr;
-    const ShotGeo &sg = a.geo[s];
-    const int r0v = sg.r0v, r02 = sg.r02, nr2 = sg.nr2;
-    const int sx0 = sg.sx0, sx1 = sg.sx1;
-    const bool src_z = MODE == FWD && iz0 <= sg.sz1 && iz0 + 3 >= sg.sz0;
-    auto issue_cur = [&](int k) {  // plane x = x0 - 4 + k
-      const int x = x0 - 4 + k;
-      const bool xok = x >= -HX && x < a.pnx + HX;
-      float4 *dst = s_cur + (k % NC) * W;
-      const long long ox = (long long)lz * x;
-      cp16(dst + ci, cur + (live && xok ? o_c + ox : 0), live && xok);
-      if (has_h) cp16(dst + hslot, cur + (h_ok && xok ? h_off + ox : 0), h_ok && xok);
-    };
-    auto issue_pv = [&](int j) {  // plane x = x0 + j
-      const long long o = o_c + (long long)lz * (x0 + j);
-      cp16(s_prev + (j % NP) * ZW + tid, live ? nxt + o : nxt, live);
-      cp16(s_V + (j % NP) * ZW + tid, live ? a.V + o : a.V, live);
-      if (MODE == ADJ_EXACT) {
-        cp16(s_t + (j % NP) * ZW + tid, live ? tin + o : tin, live && a.imaging);
-        cp16(s_g + (j % NP) * ZW + tid, live ? gs + o : gs, live && a.imaging);
-      }
-      if (MODE == FWD && PAS) {
-        // the interior cells' source samples of plane x0 + j (zero elsewhere)
-        const int x = x0 + j;
-        const bool xin = live && x >= a.nb && x < a.nb + a.nx;
-        const float *row = a.dsrc + s * a.dsrc_stride +
-                           ((long long)a.it * a.nx + (xin ? x - a.nb : 0)) * a.nz;
-        float *dst = reinterpret_cast<float *>(s_d + (j % NP) * ZW + tid);
+    const f2 s_wx = pk2(L.w, c.x), s_yz = pk2(c.y, c.z), s_wR = pk2(c.w, R.x);
+    const f2 s_Lyz = pk2(L.y, L.z), s_Ryz = pk2(R.y, R.z);
+    // z partners (+d, -d) of each pair, d = 1 .. 4
+    const f2 zp[2][4] = {{s_yz, ch, s_wR, lo2(R)}, {s_wR, lo2(R), s_Ryz, hi2(R)}};
+    const f2 zm[2][4] = {{s_wx, hi2(L), s_Lyz, lo2(L)}, {s_yz, cl, s_wx, hi2(L)}};
+    f2 tx2[2], tz2[2];
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const int iz = iz0 + e;
-          const bool ok = xin && iz >= a.nb && iz < a.nb + a.nz;
-          cp4(dst + e, ok ? row + (iz - a.nb) : a.dsrc, ok);
-        }
-      }
-    };
-    for (int k = 0; k < 8; k++) issue_cur(k);
+    for (int h = 0; h < 2; h++) {
+      f2 tx = mul2(mul2(kc[0], h ? ch : cl), k1);
+      f2 tz = tx;
 #pragma unroll
-    for (int b = 0; b < P; b++) {
-      if (b < nplanes) {
-        issue_cur(b + 8);
-        issue_pv(b);
+      for (int d = 1; d <= 4; d++) {
+        const float4 &xp = q[4 + d], &xm = q[4 - d];
+        const f2 xs = h ? add2(hi2(xp), hi2(xm)) : add2(lo2(xp), lo2(xm));
+        tx = add2(tx, mul2(mul2(kc[d], xs), k1));
       }
-      cp_commit();
+#pragma unroll
+      for (int d = 1; d <= 4; d++)
+        tz = add2(tz, mul2(mul2(kc[d], add2(zp[h][d - 1], zm[h][d - 1])), k1));
+      tx2[h] = tx;
+      tz2[h] = tz;
     }
-    float4 q[9];
-    for (int i = 0; i < nplanes; i++) {
-      const int x = x0 + i;
-      // ADJ_REF imaging operands of this plane, loaded before the stencil so
-      // their latency hides behind it
-      double rw[4];
-      float rt[4], rg[4];
-      const bool img = MODE == ADJ_REF && a.imaging && live && x >= a.nb && x < a.nb + a.nx;
-      if (MODE == ADJ_REF) {
+    div4_sum(tx2, tz2, a.divx, a.divz, a.xlo, a.xhi, !(lz_any && lx_ok), t2);
+  }
+  float4 term4 = join2(t2[0], t2[1]);
+  if (!(lz_full && lx_ok)) {
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const int iz = iz0 + e;
-          rw[e] = 0.;
-          rt[e] = rg[e] = 0.f;
-          if (img && iz >= a.nb && iz < a.nb + a.nz) {
-            const size_t k = (size_t)(x - a.nb) * a.nz + (iz - a.nb);
-            const size_t ks = s * a.wstride + k;
-            // wave[wit+1] - 2.*wave[wit] + wave[wit-1] in double, left to right
-            rw[e] = __dadd_rn(__dsub_rn((double)a.wnext[ks], __dmul_rn(2., (double)a.wcur[ks])),
-                              (double)a.wprev[ks]);
-            rt[e] = a.m2v3[k];
-            rg[e] = gs[k];
-          }
-        }
-      }
-      if (i + P < nplanes) {
-        issue_cur(i + P + 8);
-        issue_pv(i + P);
-      }
-      cp_commit();
-      cp_wait<P>();
-      __syncthreads();
-      if (i == 0) {
+    for (int e = 0; e < 4; e++)
+      if (!(lz_any && lx_ok && iz0 + e < a.pnz - 4)) set_el(term4, e, 0.f);
+  }
+  if (MODE == FWD && PAS) {
+    // gradient_pas_av (wave_fwigradient.c:732-737): the interior's source
+    // sample; its update covers the stencil's cells only, so none is
+    // added on the 4-cell rim
 #pragma unroll
-        for (int k = 0; k < 8; k++) q[k] = s_cur[k * W + ci];
-      }
-      q[8] = s_cur[((i + 8) % NC) * W + ci];
-      const float4 *pl = s_cur + ((i + 4) % NC) * W;
-      if (live) {
-        const float4 c = q[4];
-        const float4 L = pl[ci - 1], R = pl[ci + 1];
-        const float4 pv = s_prev[(i % NP) * ZW + tid];
-        const float4 V4 = s_V[(i % NP) * ZW + tid];
-        const float4 dv = (MODE == FWD && PAS) ? s_d[(i % NP) * ZW + tid]
-                                               : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float bxf = a.bx[x];
-        const bool lx_ok = x >= 4 && x < a.pnx - 4;
-        const long long o = o_c + (long long)lz * x;
-        // receivers read the field before the update (wave_fwimodeling.c:76-79)
-        int rir = -1;
-        if (rec_row) {
-          const int d = x - r0v;
-          if (d >= 0) {
-            const int ir = a.drv == 1 ? d : (d % a.drv == 0 ? d / a.drv : -1);
-            if (ir >= 0 && ir < nr2) rir = r02 + ir;
-          }
-        }
-        const bool src_here = src_z && x >= sx0 && x <= sx1;
-        if (MODE == FWD && rir >= 0 && a.rec)
-          a.rec[((size_t)s * a.nt + a.it) * a.nr + rir] = el(c, a.rz - iz0);
-        const bool interior = x >= a.nb && x < a.nb + a.nx;
-        if (MODE == FWD && a.snap && interior) {
-#pragma unroll
-          for (int e = 0; e < 4; e++) {
-            const int iz = iz0 + e;
-            if (iz >= a.nb && iz < a.nb + a.nz)
-              a.snap[s * a.snap_stride + (size_t)(x - a.nb) * a.nz + (iz - a.nb)] = el(c, e);
-          }
-        }
-        float4 term4, res4;
-        float txs[4], tzs[4], qx[4], qz[4];
-        {
-          // the x and z sums of the 8th-order Laplacian in the reference's
-          // order, cells (0, 1) and (2, 3) of the float4 per f32x2 op; the
-          // z neighbours at odd distances are the float4s shifted by one cell
-          const f2 k1 = pk2(a.one, a.one);
-          const f2 kc[5] = {pk2(a.c0, a.c0), pk2(a.c1, a.c1), pk2(a.c2, a.c2), pk2(a.c3, a.c3),
-                            pk2(a.c4, a.c4)};
-          const f2 cl = lo2(c), ch = hi2(c);
-          const f2 s_wx = pk2(L.w, c.x), s_yz = pk2(c.y, c.z), s_wR = pk2(c.w, R.x);
-          const f2 s_Lyz = pk2(L.y, L.z), s_Ryz = pk2(R.y, R.z);
-          // z partners (+d, -d) of each pair, d = 1 .. 4
-          const f2 zp[2][4] = {{s_yz, ch, s_wR, lo2(R)}, {s_wR, lo2(R), s_Ryz, hi2(R)}};
-          const f2 zm[2][4] = {{s_wx, hi2(L), s_Lyz, lo2(L)}, {s_yz, cl, s_wx, hi2(L)}};
-          f2 tx2[2], tz2[2];
-#pragma unroll
-          for (int h = 0; h < 2; h++) {
-            const f2 cv2 = h ? ch : cl;
-            f2 tx = mul2(mul2(kc[0], cv2), k1);
-#pragma unroll
-            for (int d = 1; d <= 4; d++) {
-              const f2 xs = h ? add2(hi2(q[4 + d]), hi2(q[4 - d])) : add2(lo2(q[4 + d]), lo2(q[4 - d]));
-              tx = add2(tx, mul2(mul2(kc[d], xs), k1));
-            }
-            f2 tz = mul2(mul2(kc[0], cv2), k1);
-#pragma unroll
-            for (int d = 1; d <= 4; d++)
-              tz = add2(tz, mul2(mul2(kc[d], add2(zp[h][d - 1], zm[h][d - 1])), k1));
-            tx2[h] = tx;
-            tz2[h] = tz;
-          }
-          const float4 tx4 = join2(tx2[0], tx2[1]), tz4 = join2(tz2[0], tz2[1]);
-#pragma unroll
-          for (int e = 0; e < 4; e++) {
-            const bool lap = lz_ok[e] && lx_ok;  // skipped cells vote with zeros
-            txs[e] = lap ? el(tx4, e) : 0.f;
-            tzs[e] = lap ? el(tz4, e) : 0.f;
-          }
-        }
-        div4x2(txs, tzs, a.divx, a.divz, __activemask(), qx, qz);
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const int iz = iz0 + e;
-          float t = (lz_ok[e] && lx_ok) ? fadd(qx[e], qz[e]) : 0.f;
-          if (MODE == FWD && PAS) {
-            // gradient_pas_av (wave_fwigradient.c:732-737): the interior's source
-            // sample; its update covers the stencil's cells only, so none is
-            // added on the 4-cell rim
-            if (lz_ok[e] && lx_ok && iz >= a.nb && iz < a.nb + a.nz && x >= a.nb &&
-                x < a.nb + a.nx)
-              t = fadd(t, el(dv, e));
-          } else if (MODE == FWD) {
-            if (src_here)
-              for (int k = 0; k < sg.nsrc; k++)
-                if (sg.scell[k] == ((x << 16) | iz)) t = fadd(t, fmul(sg.sw[k], a.wav[a.it]));
-          } else if (rir >= 0 && iz == a.rz) {
-            t = fadd(t, a.res[((size_t)s * a.nt + a.it) * a.nr + rir]);
-          }
-          set_el(term4, e, t);
-        }
-        {
-          // b = S(a_{k-1} as stored): z faces then x faces (apply_sponge);
-          // 2 c as c + c (the same bits, and no product to fuse into the
-          // subtraction)
-          const f2 k1 = pk2(a.one, a.one), bx2 = pk2(bxf, bxf);
-          f2 r2[2];
-#pragma unroll
-          for (int h = 0; h < 2; h++) {
-            const f2 bz2 = pk2(bzf[2 * h], bzf[2 * h + 1]);
-            const f2 cv2 = h ? hi2(c) : lo2(c);
-            const f2 p = mul2(mul2(bx2, mul2(bz2, h ? hi2(pv) : lo2(pv))), k1);
-            const f2 vt = mul2(mul2(h ? hi2(V4) : lo2(V4), h ? hi2(term4) : lo2(term4)), k1);
-            const f2 v = add2(sub2(add2(cv2, cv2), p), vt);
-            r2[h] = mul2(bx2, mul2(bz2, v));
-          }
-          res4 = join2(r2[0], r2[1]);
-#pragma unroll
-          for (int e = 0; e < 4; e++)
-            if (!zin[e]) set_el(res4, e, 0.f);
-        }
-        *reinterpret_cast<float4 *>(nxt + o) = res4;
-        if (MODE == FWD && a.tout)
-          *reinterpret_cast<float4 *>(a.tout + s * a.tout_stride + o) = term4;
-        if (MODE == ADJ_EXACT && a.imaging) {
-          // dJ/dV accumulates phi_n * term_n (divided by V at the end)
-          const float4 tf = s_t[(i % NP) * ZW + tid];
-          const float4 g4 = s_g[(i % NP) * ZW + tid];  // read P planes ahead (cp.async)
-          const f2 k1 = pk2(a.one, a.one);
-          const float4 gacc = join2(add2(lo2(g4), mul2(mul2(lo2(c), lo2(tf)), k1)),
-                                    add2(hi2(g4), mul2(mul2(hi2(c), hi2(tf)), k1)));
-          *reinterpret_cast<float4 *>(gs + o) = gacc;
-        }
-        if (MODE == ADJ_REF && img) {
-          // gradient_av (wave_fwigradient.c:221-230): the C expression in
-          // double, unfused, added to the float gradient
-#pragma unroll
-          for (int e = 0; e < 4; e++) {
-            const int iz = iz0 + e;
-            if (iz >= a.nb && iz < a.nb + a.nz) {
-              const size_t k = (size_t)(x - a.nb) * a.nz + (iz - a.nb);
-              const double gsum = __dmul_rn(__dmul_rn(__ddiv_rn(rw[e], (double)a.wdt2),
-                                                      (double)el(c, e)),
-                                            (double)rt[e]);
-              gs[k] = __double2float_rn(__dadd_rn((double)rg[e], gsum));
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < 8; k++) q[k] = q[k + 1];
+    for (int e = 0; e < 4; e++) {
+      const int iz = iz0 + e;
+      if (iz >= 4 && iz < a.pnz - 4 && lx_ok && xin && iz >= a.nb && iz < a.nb + a.nz)
+        set_el(term4, e, fadd(el(term4, e), dv[e]));
     }
-    cp_wait_all();
-    __syncthreads();
+  } else if (MODE == FWD) {
+    if (src_z && x >= sg.sx0 && x <= sg.sx1) {
+      const float w = a.wav[a.it];
+#pragma unroll
+      for (int e = 0; e < 4; e++)
+        for (int k = 0; k < sg.nsrc; k++)
+          if (sg.scell[k] == ((x << 16) | (iz0 + e)))
+            set_el(term4, e, fadd(el(term4, e), fmul(sg.sw[k], w)));
+    }
+  } else if (rir >= 0) {
+    const float r = a.res[((size_t)s * a.nt + a.it) * a.nr + rir];
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+      if (iz0 + e == a.rz) set_el(term4, e, fadd(el(term4, e), r));
+  }
+  {
+    // b = S(a_{k-1} as stored): z faces then x faces (apply_sponge);
+    // 2 c as c + c (the same bits, and no product to fuse into the
+    // subtraction).  Cells beyond pnz and pnx stay zero: every operand
+    // is zero there
+    const f2 bx2 = pk2(bxf, bxf);
+    f2 r2[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const f2 bz2 = h ? hi2(bz4) : lo2(bz4);
+      const f2 cv2 = h ? ch : cl;
+      const f2 p = mul2(mul2(bx2, mul2(bz2, h ? hi2(p4) : lo2(p4))), k1);
+      const f2 vt = mul2(mul2(h ? hi2(V4) : lo2(V4), h ? hi2(term4) : lo2(term4)), k1);
+      const f2 v = add2(sub2(add2(cv2, cv2), p), vt);
+      r2[h] = mul2(bx2, mul2(bz2, v));
+    }
+    *reinterpret_cast<float4 *>(pn) = join2(r2[0], r2[1]);
+  }
+  if (MODE == FWD && a.tout) __stcs(reinterpret_cast<float4 *>(po), term4);
+  if (MODE == ADJ_EXACT) {
+    // dJ/dV accumulates phi_n * term_n (divided by V at the end)
+    *reinterpret_cast<float4 *>(pg) =
+        join2(add2(lo2(g4), mul2(mul2(cl, lo2(tf)), k1)),
+              add2(hi2(g4), mul2(mul2(ch, hi2(tf)), k1)));
+  }
+  if (MODE == ADJ_REF && img) {
+    // gradient_av (wave_fwigradient.c:221-230): the C expression in
+    // double, unfused, added to the float gradient
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      const int iz = iz0 + e;
+      if (iz >= a.nb && iz < a.nb + a.nz) {
+        const size_t k = (size_t)(x - a.nb) * a.nz + (iz - a.nb);
+        const double gsum = __dmul_rn(__dmul_rn(__ddiv_rn(rw[e], (double)a.wdt2),
+                                                (double)el(c, e)),
+                                      (double)rt[e]);
+        gs[k] = __double2float_rn(__dadd_rn((double)rg[e], gsum));
+      }
+    }
   }
 }
 
@@ -871,18 +779,6 @@ __global__ void fastdiv_check_kernel(float d, float zh, float zl, float scale) {
   if (__float_as_uint(q) != __float_as_uint(__fdiv_rn(x, d))) atomicAdd(&fastdiv_bad, 1u);
 }
 
-// div_small against __fdiv_rn for every float with bits in [1, umin), both signs
-__global__ void smalldiv_check_kernel(DivC c) {
-  const unsigned int stride = gridDim.x * blockDim.x;
-  unsigned int bad = 0;
-  for (unsigned int u = 1 + blockIdx.x * blockDim.x + threadIdx.x; u < c.umin; u += stride) {
-    const float x = __uint_as_float(u), y = -x;
-    bad += __float_as_uint(div_small(x, c)) != __float_as_uint(__fdiv_rn(x, c.d));
-    bad += __float_as_uint(div_small(y, c)) != __float_as_uint(__fdiv_rn(y, c.d));
-  }
-  if (bad) atomicAdd(&fastdiv_bad, bad);
-}
-
 // DivC for d (cached per process: the result depends on d only).
 static int prepare_div(float d, DivC &c) {
   static std::mutex mu;
@@ -896,11 +792,11 @@ static int prepare_div(float d, DivC &c) {
     return PW_OK;
   }
   c.d = d;
-  c.ok = 0;
+  c.dd = d;
+  c.rd = 1.0 / (double)d;
   c.zh = c.zl = 0.f;
   c.xmin = 1.f;
   c.xmax = 0.f;
-  c.umin = c.uspan = c.umax = 0;
   if (d > 0.f && std::isfinite(d)) {
     // zh: the float nearest 1/d (float x float products are exact in double,
     // and 1 - zh*d is exact by Sterbenz's lemma)
@@ -924,35 +820,23 @@ static int prepare_div(float d, DivC &c) {
     lo *= 4;
     const double hi = std::min({fmax / 4 / zh, fmax / 4 * d, fmax});  // finite numerators only
     if (lo * 4 < hi) {
-      c.zh = zh;
-      c.zl = zl;
-      c.xmin = (float)lo;
-      c.xmax = (float)hi;
-      memcpy(&c.umin, &c.xmin, 4);
-      memcpy(&c.umax, &c.xmax, 4);
-      c.uspan = c.umax - c.umin;
-      c.sup = std::ldexp(1.f, DIV_SMALL_K);
-      c.sdn = std::ldexp(1.f, -DIV_SMALL_K);
-      c.sgrid = std::ldexp(1.f, 149 - DIV_SMALL_K);
-      // x in (0, xmin) scales into [2^(K-149), xmin * 2^K], inside [xmin, xmax]
-      const bool small_ok = lo <= std::ldexp(1.0, DIV_SMALL_K - 149) &&
-                            lo * std::ldexp(1.0, DIV_SMALL_K) <= hi;
       const double scale = std::ldexp(1.0, (int)std::ceil(std::log2(lo)));
       unsigned int bad = 0;
       PW_CUDA(cudaMemcpyToSymbol(fastdiv_bad, &bad, sizeof bad));
       fastdiv_check_kernel<<<(1u << 23) / 256, 256>>>(d, zh, zl, (float)scale);
       PW_CUDA(cudaGetLastError());
-      if (small_ok) {
-        smalldiv_check_kernel<<<4 * 148, 256>>>(c);
-        PW_CUDA(cudaGetLastError());
-      }
       PW_CUDA(cudaMemcpyFromSymbol(&bad, fastdiv_bad, sizeof bad));
-      c.ok = small_ok && bad == 0;
+      if (bad == 0) {
+        c.zh = zh;
+        c.zl = zl;
+        c.xmin = (float)lo;
+        c.xmax = (float)hi;
+      }
     }
   }
   if (getenv("PW_PFWI_VERBOSE"))
-    fprintf(stderr, "pfwi: division by %.9g: zh %.9g zl %.9g range [%.3g, %.3g] fast %d\n", d,
-            c.zh, c.zl, c.xmin, c.xmax, c.ok);
+    fprintf(stderr, "pfwi: division by %.9g: zh %.9g zl %.9g range [%.3g, %.3g]\n", d, c.zh, c.zl,
+            c.xmin, c.xmax);
   cache[key] = c;
   return PW_OK;
 }
@@ -965,8 +849,6 @@ struct Setup {
   int nr, rz, drv, sz;
   std::vector<ShotGeo> geo;
   std::vector<float> bz, bx;
-  int zw, ztiles, nsm;
-  size_t smem;
 };
 
 // passive: distributed sources (pfwi mode 4) -- no point source per shot
@@ -998,6 +880,7 @@ static int setup(const pw_fwi_args *a, Setup &S, bool passive = false) {
   };
   axis(S.pnz, S.bz);
   axis(S.pnx, S.bx);
+  S.bz.resize(round_up(S.pnz, 4), 1.f);  // read four at a time
   const float dx = a->dx;
   const int ds_v = (int)(a->ds / dx + 0.5);
   const int s0_v = (int)(a->os / dx + 0.5 + nb);
@@ -1039,67 +922,30 @@ static int setup(const pw_fwi_args *a, Setup &S, bool passive = false) {
     PW_TRY(source_map(sx, S.sz, S.pnz, S.pnx, g));
   }
   PW_CHECK(S.rz >= 4 && S.rz < S.pnz - 4, PW_ERR_SHAPE, "receiver depth in the zero border");
-  // tile: one z segment of ZW float4 (whole column when it fits)
-  const int nz4 = ceil_div(S.pnz, 4);
-  S.zw = nz4 <= 64 ? 64 : 128;
-  const int ztiles = ceil_div(nz4, S.zw);
-  int dev = 0, nsm = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  S.ztiles = ztiles;
-  S.nsm = nsm;
-  if (getenv("PW_PFWI_VERBOSE"))
-    fprintf(stderr, "pfwi plan: padded %d x %d, ZW=%d ztiles=%d\n", S.pnz, S.pnx, S.zw, S.ztiles);
+  if (getenv("PW_PFWI_VERBOSE")) {
+    // depth class of the padded grid: columns of up to 64 or 128 float4, and
+    // how many such segments a column has (the step kernel's lanes cross
+    // columns and use neither)
+    const int nz4 = ceil_div(S.pnz, 4), zw = nz4 <= 64 ? 64 : 128;
+    fprintf(stderr, "pfwi plan: padded %d x %d, ZW=%d ztiles=%d\n", S.pnz, S.pnx, zw,
+            ceil_div(nz4, zw));
+  }
   return PW_OK;
 }
 
-// prefetch depth (planes): one plane ahead is enough once the x chunks are
-// short, and the smaller ring lets more CTAs share an SM (32 shots of 420 x
-// 720 at nt 500: forward 36.3 -> 33.0 ms, exact gradient 79.5 -> 70.7 ms
-// against 3 planes)
-constexpr int PFP = 1;
-
-static size_t smem_for(int zw, int mode) {
-  return sizeof(float4) * ((size_t)(PFP + 10) * (zw + 2) + (size_t)(mode == ADJ_EXACT ? 4 : 2) *
-                                                               (PFP + 2) * zw);
-}
-
-template <int ZW, int MODE, bool PAS = false>
-static int launch_one(const Setup &S, const PfArgs &p, cudaStream_t st) {
-  // the forward step with passive sources adds a ring of source planes
-  const size_t smem = smem_for(ZW, MODE) + (PAS ? (size_t)(PFP + 2) * ZW * sizeof(float4) : 0);
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(pf_step_kernel<ZW, PFP, MODE, PAS>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    attr = true;
-  }
-  // x planes per CTA: long enough to amortise the 8-plane prologue, short
-  // enough that shots x chunks x z tiles give every SM 12 CTAs (about three
-  // waves of the 4 that fit).  Small batches go down to one plane per CTA:
-  // a step is then a few dependent plane updates instead of a long chain
-  // (the passive demos' grid, 3 shots: 175 ms per gradient at 16 planes,
-  // 46 ms at 1), the re-read halo planes staying in L2; 32 shots of 420 x
-  // 720 run 8 planes (2.94 gradients/s, 2.69 at 16)
-  int xch = 128;
-  while (xch > 1 && (long long)p.nshots * S.ztiles * ceil_div(S.pnx, xch) < 12LL * S.nsm) xch /= 2;
-  const dim3 grid(p.nshots, ceil_div(S.pnx, xch), S.ztiles);
-  pf_step_kernel<ZW, PFP, MODE, PAS><<<grid, ZW, smem, st>>>(p, xch);
-  PW_CUDA(cudaGetLastError());
+template <int MODE, bool PAS = false>
+static int launch_one(const Setup &S, const PfArgs &p, int nshots, cudaStream_t st) {
+  const long long lanes = (long long)p.nz4 * ceil_div(S.pnx, PF_XW);
+  const dim3 grid((unsigned)ceil_div(lanes, 32), (unsigned)nshots);
+  PW_CUDA(launch_pdl(pf_step_kernel<MODE, PAS>, grid, dim3(32 * PF_XW), 0, st, p));
   return PW_OK;
 }
 
-static int launch(const Setup &S, const PfArgs &p, int mode, cudaStream_t st) {
-  if (mode == FWD && p.dsrc)
-    return S.zw == 64 ? launch_one<64, FWD, true>(S, p, st) : launch_one<128, FWD, true>(S, p, st);
-  if (S.zw == 64) {
-    if (mode == FWD) return launch_one<64, FWD>(S, p, st);
-    if (mode == ADJ_REF) return launch_one<64, ADJ_REF>(S, p, st);
-    return launch_one<64, ADJ_EXACT>(S, p, st);
-  }
-  if (mode == FWD) return launch_one<128, FWD>(S, p, st);
-  if (mode == ADJ_REF) return launch_one<128, ADJ_REF>(S, p, st);
-  return launch_one<128, ADJ_EXACT>(S, p, st);
+static int launch(const Setup &S, const PfArgs &p, int mode, int nshots, cudaStream_t st) {
+  if (mode == FWD)
+    return p.dsrc ? launch_one<FWD, true>(S, p, nshots, st) : launch_one<FWD>(S, p, nshots, st);
+  if (mode == ADJ_REF) return launch_one<ADJ_REF>(S, p, nshots, st);
+  return launch_one<ADJ_EXACT>(S, p, nshots, st);
 }
 
 static void base_args(const Setup &S, PfArgs &p) {
@@ -1112,16 +958,34 @@ static void base_args(const Setup &S, PfArgs &p) {
   p.nx = S.a.nx;
   const float c0 = -205. / 72, c1 = 8. / 5, c2 = -1. / 5, c3 = 8. / 315, c4 = -1. / 560;
   p.c0 = c0; p.c1 = c1; p.c2 = c2; p.c3 = c3; p.c4 = c4;
-  p.dx2 = S.a.dx * S.a.dx;
-  p.dz2 = S.a.dz * S.a.dz;
   p.one = 1.f;
   p.divx = S.divx;
   p.divz = S.divz;
+  p.xlo = std::max(S.divx.xmin, S.divz.xmin);
+  p.xhi = std::min(S.divx.xmax, S.divz.xmax);
   p.nt = S.a.nt;
   p.rz = S.rz;
   p.drv = S.drv;
   p.nr = S.nr;
-  p.fstride = S.fstride;
+  p.fstep = S.fstride;
+  p.nz4 = ceil_div(S.pnz, 4);
+  // m = ceil(2^(32 + k) / nz4) with 2^k >= nz4 divides every n < 2^31 exactly
+  // where m fits 32 bits (nz4 > 1); with nz4 = 1 the halved form is n itself
+  int k = 0;
+  while ((1 << k) < p.nz4) k++;
+  if (k == 0) {
+    p.div_m = 0xffffffffu;
+    p.div_s = 0;
+  } else {
+    p.div_m = (unsigned)(((1ull << (31 + k)) + p.nz4 - 1) / p.nz4);
+    p.div_s = k - 1;
+  }
+  p.src_z0 = 1 << 30;
+  p.src_z1 = -1;
+  for (const ShotGeo &g : S.geo) {
+    p.src_z0 = std::min(p.src_z0, g.sz0);
+    p.src_z1 = std::max(p.src_z1, g.sz1);
+  }
 }
 
 }  // namespace pf
@@ -1301,25 +1165,18 @@ extern "C" int pw_pfwi_forward(const pw_fwi_args *a, const float *vel, const flo
   long long launches = 0;
   for (int s0 = 0; s0 < ns; s0 += nsb) {
     const int nb_ = std::min(nsb, ns - s0);
-    float *A[MAXS], *B[MAXS];
-    for (int s = 0; s < nb_; s++) {
-      A[s] = at<float>(base, o_A) + (size_t)s * S.fstride;
-      B[s] = at<float>(base, o_B) + (size_t)s * S.fstride;
-    }
-    PW_CUDA(cudaMemsetAsync(base + o_A, 0, (size_t)nsb * S.fstride * 4, st));
-    PW_CUDA(cudaMemsetAsync(base + o_B, 0, (size_t)nsb * S.fstride * 4, st));
-    p.nshots = nb_;
+    float *A = at<float>(base, o_A), *B = at<float>(base, o_B);
+    PW_CUDA(cudaMemsetAsync(A, 0, (size_t)nsb * S.fstride * 4, st));
+    PW_CUDA(cudaMemsetAsync(B, 0, (size_t)nsb * S.fstride * 4, st));
     p.geo = at<ShotGeo>(base, o_geo) + s0;
     p.rec = rec + (size_t)s0 * nt * nr;
     for (int it = 0; it < nt; it++) {
       p.it = it;
-      for (int s = 0; s < nb_; s++) {
-        p.cur[s] = A[s];
-        p.nxt[s] = B[s];
-      }
-      PW_TRY(launch(S, p, FWD, st));
+      p.cur = A;
+      p.nxt = B;
+      PW_TRY(launch(S, p, FWD, nb_, st));
       launches++;
-      for (int s = 0; s < nb_; s++) std::swap(A[s], B[s]);
+      std::swap(A, B);
     }
   }
   timer.stop();
@@ -1563,28 +1420,25 @@ static int gradient_impl(const pw_fwi_args *a, int mode, const float *vel, const
   timer.start();
   for (int s0 = 0; s0 < ns; s0 += nsb) {
     const int nb_ = std::min(nsb, ns - s0);
-    float *A[MAXS], *B[MAXS];
+    // the shots' wavefield pairs, `stride` floats apart; a step swaps the pair
+    float *A, *B;
     auto reset = [&]() -> int {
-      for (int s = 0; s < nb_; s++) {
-        A[s] = at<float>(base, o_A) + s * fs;
-        B[s] = at<float>(base, o_B) + s * fs;
-      }
-      PW_CUDA(cudaMemsetAsync(base + o_A, 0, (size_t)nsb * fs * 4, st));
-      PW_CUDA(cudaMemsetAsync(base + o_B, 0, (size_t)nsb * fs * 4, st));
+      A = at<float>(base, o_A);
+      B = at<float>(base, o_B);
+      PW_CUDA(cudaMemsetAsync(A, 0, (size_t)nsb * fs * 4, st));
+      PW_CUDA(cudaMemsetAsync(B, 0, (size_t)nsb * fs * 4, st));
       return PW_OK;
     };
-    auto step = [&](int mode_, int it) -> int {
+    auto step = [&](int mode_, int it, float *&cur, float *&nxt, size_t stride) -> int {
       p.it = it;
-      for (int s = 0; s < nb_; s++) {
-        p.cur[s] = A[s];
-        p.nxt[s] = B[s];
-      }
-      PW_TRY(launch(S, p, mode_, st));
+      p.cur = cur;
+      p.nxt = nxt;
+      p.fstep = (long long)stride;
+      PW_TRY(launch(S, p, mode_, nb_, st));
       launches++;
-      for (int s = 0; s < nb_; s++) std::swap(A[s], B[s]);
+      std::swap(cur, nxt);
       return PW_OK;
     };
-    p.nshots = nb_;
     p.geo = at<ShotGeo>(base, o_geo) + s0;
     p.dsrc = d_dsrc ? d_dsrc + (size_t)s0 * nsrcf : nullptr;
     p.dsrc_stride = (long long)nsrcf;
@@ -1605,14 +1459,14 @@ static int gradient_impl(const pw_fwi_args *a, int mode, const float *vel, const
         const int m = it / k;
         for (int s = 0; s < nb_; s++) {
           float *c = ck + ((size_t)s * nck + m) * 2 * fs;
-          PW_CUDA(cudaMemcpyAsync(c, A[s], fs * 4, cudaMemcpyDeviceToDevice, st));
-          PW_CUDA(cudaMemcpyAsync(c + fs, B[s], fs * 4, cudaMemcpyDeviceToDevice, st));
+          PW_CUDA(cudaMemcpyAsync(c, A + s * fs, fs * 4, cudaMemcpyDeviceToDevice, st));
+          PW_CUDA(cudaMemcpyAsync(c + fs, B + s * fs, fs * 4, cudaMemcpyDeviceToDevice, st));
         }
       }
       p.snap = (!exact && it % interval == 0) ? snap + (size_t)(it / interval) * nvel : nullptr;
       // the last segment's terms, which the backward pass reads first
       p.tout = it >= n_last ? tb + (size_t)(it - n_last) * fs : nullptr;
-      PW_TRY(step(FWD, it));
+      PW_TRY(step(FWD, it, A, B, fs));
     }
     p.rec = nullptr;
     p.snap = nullptr;
@@ -1642,62 +1496,29 @@ static int gradient_impl(const pw_fwi_args *a, int mode, const float *vel, const
           p.wcur = snap + (size_t)wit * nvel;
           p.wnext = snap + (size_t)(wit + 1) * nvel;
         }
-        PW_TRY(step(ADJ_REF, it));
+        PW_TRY(step(ADJ_REF, it, A, B, fs));
       }
     } else {
-      // ---- backward by segments: restore checkpoint, recompute the forward
-      // terms of the segment, run the exact adjoint over it
-      float *PA[MAXS], *PB[MAXS];
-      for (int s = 0; s < nb_; s++) {
-        PA[s] = at<float>(base, o_A) + s * fs;  // reused: adjoint after the forward
-        PB[s] = at<float>(base, o_B) + s * fs;
-      }
-      // the adjoint needs its own pair; the forward recompute restores from
-      // the checkpoints into the segment buffer's first two slots
-      PW_CUDA(cudaMemsetAsync(base + o_A, 0, (size_t)nsb * fs * 4, st));
-      PW_CUDA(cudaMemsetAsync(base + o_B, 0, (size_t)nsb * fs * 4, st));
-      float *adjA[MAXS], *adjB[MAXS];
-      for (int s = 0; s < nb_; s++) {
-        adjA[s] = PA[s];
-        adjB[s] = PB[s];
-      }
+      // ---- backward by segments: recompute the forward terms of the segment
+      // from its checkpoint, run the exact adjoint over it
+      PW_TRY(reset());  // the adjoint reuses the forward pair
       p.tout_stride = (long long)k * fs;
       p.tin_stride = (long long)k * fs;
       for (int m = nck - 1; m >= 0; m--) {
         const int n0 = m * k, n1 = std::min(nt, n0 + k);
-        // recompute: fwd pair lives in checkpoint m (overwritten, no longer needed)
-        float *FA[MAXS], *FB[MAXS];
-        for (int s = 0; s < nb_; s++) {
-          FA[s] = ck + ((size_t)s * nck + m) * 2 * fs;
-          FB[s] = FA[s] + fs;
-        }
+        // the forward pair lives in checkpoint m (overwritten, no longer needed)
+        float *FA = ck + (size_t)m * 2 * fs, *FB = FA + fs;
         for (int n = n0; n < n1 && m < nck - 1; n++) {  // the last segment is kept
-          p.it = n;
-          for (int s = 0; s < nb_; s++) {
-            p.cur[s] = FA[s];
-            p.nxt[s] = FB[s];
-          }
           p.tout = tb + (size_t)(n - n0) * fs;
-          PW_TRY(launch(S, p, FWD, st));
-          launches++;
-          for (int s = 0; s < nb_; s++) std::swap(FA[s], FB[s]);
+          PW_TRY(step(FWD, n, FA, FB, (size_t)nck * 2 * fs));
         }
         p.tout = nullptr;
         for (int n = n1 - 1; n >= n0; n--) {
-          p.it = n;
-          for (int s = 0; s < nb_; s++) {
-            p.cur[s] = adjA[s];
-            p.nxt[s] = adjB[s];
-          }
           p.tin = tb + (size_t)(n - n0) * fs;
-          p.imaging = 1;
-          PW_TRY(launch(S, p, ADJ_EXACT, st));
-          launches++;
-          for (int s = 0; s < nb_; s++) std::swap(adjA[s], adjB[s]);
+          PW_TRY(step(ADJ_EXACT, n, A, B, fs));
         }
       }
       p.tin = nullptr;
-      p.imaging = 0;
     }
     if (sliced) {
       sum_slices_kernel<<<592, 256, 0, st>>>(gslices, nb_, (long long)gslice, gtotal);

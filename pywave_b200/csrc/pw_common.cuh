@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 #include <mutex>
 
@@ -125,6 +126,24 @@ class LoopTimer {
 // holds the device's workspace lock.
 void release_fft_plans();
 
+// Launch that may overlap its prologue with the end of the stream's previous
+// kernel (the kernel calls pdl_wait before it touches that kernel's data).
+template <class... P, class... A>
+inline cudaError_t launch_pdl(void (*fn)(P...), dim3 grid, dim3 block, size_t smem,
+                              cudaStream_t st, A &&...args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, fn, std::forward<A>(args)...);
+}
+
 // Copy helper honouring PW_HOST_PTRS.
 int to_device(void *dst, const void *src, size_t bytes, bool host, cudaStream_t s);
 int to_host(void *dst, const void *src, size_t bytes, bool host, cudaStream_t s);
@@ -139,6 +158,15 @@ __device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b)
 __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdiv_rn(a, b); }
+
+// Programmatic dependent launch: pdl_wait() returns when every kernel this
+// one depends on has completed (its writes visible), pdl_launch() lets the
+// next kernel of the stream start its prologue once every block has issued
+// it.  Kernels call pdl_wait() before pdl_launch(), so when the next kernel
+// starts everything before this one has completed.  Both do nothing in a
+// kernel launched without the attribute (launch_pdl sets it).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;"); }
 
 // Packed pairs of floats for sm_100's f32x2 pipe: add / sub / mul.rn.f32x2
 // round each lane exactly as the scalar __fadd_rn / __fsub_rn / __fmul_rn.
