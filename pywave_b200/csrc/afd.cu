@@ -5,25 +5,21 @@
 // of the reference's fdm2d / fdm time loop (pywave/src/wave_fdm.c:551-662,
 // 209-354) with its exact float evaluation order (no FMA contraction).
 //
-// Kernel axes.  z is contiguous; x is the tile axis; y is the marched axis.
+// Kernel axes.  z is contiguous, then x, then y (the warp-tile kernels march y).
 // 3-D maps (z,x,y) to the model's (z,x,y).  2-D maps the model's x to the
-// marched axis y and uses a dummy x axis of extent 1, so one field layout
+// y and uses a dummy x axis of extent 1, so one field layout
 // serves both.  Field layout: a zero-haloed array
 //   off(iz,ix,iy) = (iz + HZ) + sx*(ix + hx) + sy*(iy + hy),
 // leading dimension a multiple of 32 floats; each thread owns one aligned
 // float4 of 4 consecutive z cells.  Halo cells are never written and stay
 // zero: that is the reference's zero border beyond the expanded grid.
 //
-// Kernels.  Each thread owns one float4 of z cells and marches it along y
-// with a 5-deep register queue of its own cells (the y neighbours).  3-D runs
-// use tile_kernel: a warp owns an 8-slot x 4-column patch and stages it (with
-// its z and x halo) per plane in a private cp.async ring in shared memory,
-// together with each lane's B and vv cells, several planes ahead; lanes read
-// their z / x neighbours there after a warp-level sync only.  2-D runs (no x
-// neighbours) use march_kernel: z neighbours by warp shuffle, the leading
-// plane, B and vv by a per-thread cp.async ring.  The TRI image of G receiver
-// groups is formed by image_kernel after each imaging step (3-D) or by
-// shuffles between the groups' lanes (2-D).
+// Kernels.  2-D runs that fit a thread-block cluster's shared memory take
+// resident_kernel (every step in one launch); the other 2-D runs and all 3-D
+// runs take the quad kernels, one float4 of z cells per thread and step.  The
+// warp-tile kernels, which march 3-D patches along y through shared-memory
+// rings, are kept as selectable variants (PW_AFD_TMA, PW_AFD_SPLIT, PW_AFD_NC,
+// PW_AFD_TILE_G<G>); their TRI images are formed by image_kernel.
 //
 // Two buffers per wavefield: at step k the kernel reads A = u_k and B =
 // u_{k-1} (as stored, tapered once) and overwrites B with u_{k+1}.  The
@@ -64,11 +60,12 @@ __host__ __device__ inline long long foff(const Geo &g, int iz, int ix, int iy) 
 
 struct StepArgs {
   Geo g;
-  int ych;  // planes per CTA along y
   int ngroups;
-  int S, ZS, KX, nzc, WPC;  // march tile: slots per column, slots / columns per CTA, z chunks,
-                            // warps per column chunk
-  int WZ, WX;               // warp-tile kernel: warps per CTA along z and x (per group)
+  FastDiv nq;  // quad kernels: float4 per column
+  int zig;     // quad kernels: 1 = odd steps run their blocks backwards
+  // warp-tile kernels: planes per CTA along y, slots per column, z chunks, warps per CTA
+  // along z and x (per group)
+  int ych, S, nzc, WZ, WX;
   float c0, c1, c2, idx, idy, idz, k0;
   // 1.0f, as a runtime value: each packed product is multiplied by it
   // before it is added, so that a product and its add fused into one FMA
@@ -84,6 +81,9 @@ struct StepArgs {
   int it, nt;
   int ns;
   int sz[MAXSRC], sx[MAXSRC], sy[MAXSRC];
+  // quad kernels: float4s with a source cell have iz0 in [sbz, sbz + sbzn] and y in
+  // [sby, sby + sbyn] (empty ranges without sources)
+  int sbz, sbzn, sby, sbyn;
   const float *rick;  // [ns][nt]
   int rz, rx0, ry0, nrx, nry;  // receivers: row rz, x in [rx0,rx0+nrx), y in [ry0,ry0+nry)
   const float *tri_dat;        // [nt][nry][nrx]
@@ -117,7 +117,7 @@ template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// Two cells per f32x2 op for the march and resident kernels (pk2 helpers;
+// Two cells per f32x2 op for the quad and resident kernels (pk2 helpers;
 // k1 is the runtime 1.0 of StepArgs::one).  lap_quad: the 4th-order
 // Laplacian of the float4 c in the reference's order (y, then x when XT,
 // then z terms), with (Lz, Lw) the two cells below c and (Rx, Ry) the two
@@ -185,229 +185,203 @@ __device__ __forceinline__ float4 taper_quad(const float4 &v, const float (&wz)[
   return join2(r[0], r[1]);
 }
 
-// March kernel: register-marched, one float4 of z cells per thread.
-//
-// Lanes map onto (z float4 slot, group) with the G receiver groups of a TRI
-// launch interleaved (lane = slot_in_warp * G + group), warps onto z chunks
-// and x columns.  Slots of one column are contiguous in memory and the x
-// stride is the column length, so a warp touches G runs of consecutive 16-B
-// cells.  Each thread marches its float4 along y:
-//   * y neighbours: a 5-deep register queue;
-//   * z neighbours: shuffles from the adjacent slot's lane (loads at warp and
-//     chunk edges);
-//   * x neighbours (3-D): loads through L1 / L2;
-//   * the leading plane of A, the previous field B and vv: cp.async copies
-//     into a per-thread ring in shared memory, MARCH_NS - 1 planes ahead.
-// A thread only reads ring slots it filled itself, so no barrier is needed;
-// the TRI image product meets the groups of a cell in adjacent lanes and is
-// formed by shuffles.  Same float evaluation order as the reference.
-constexpr int MARCH_MAXT = 512;  // threads per CTA (launch bound)
-constexpr int MARCH_NS = 4;      // ring slots per stream: MARCH_NS - 1 planes in flight
+// Quad kernels: one step for one float4 of z cells (slot) of column (ix, y),
+// every receiver group in turn, straight from global memory: 4 (2-D) or 8
+// neighbour float4s, the adjacent z pairs, the previous field; vv, the taper
+// factors and all index work are shared by the groups, and the TRI image of
+// an imaging step is formed in registers.  No march, no shared memory, no
+// barrier: neighbours come from L1 and L2, and many small independent threads
+// hide the latency.  Same float evaluation order as the reference.
+// Bound: 261^3 time reversal of 4 groups, L2 to L1 traffic (2.3 GB per step
+// at 215 us; without any neighbour load it takes 180, the 925 MB of fields at
+// the measured copy rate 143); 261^3 forward 56 us (56 without neighbour
+// loads); 141^3 and the 2-D sections, which stay in L2, launch and load
+// latency.  Measured per step against the kernels before (warp patches that
+// march y through shared-memory rings; 2-D columns marched through a
+// per-thread ring): 261^3, 4 groups 231 -> 215 us (183 instructions per
+// float4 instead of 263); 261^3 forward 103 -> 56; 141^3 forward 25 -> 9.6;
+// 561 x 1561 forward 8.2 -> 3.6; 12 uneven shots 44.7 -> 29.  Marching up to 8
+// planes per thread with the y neighbours in registers: 217 / 77 / 13 us on
+// the 3-D grids; CTAs of 4 x 4 columns 250 / 84 / 12.8, of 8 slots x 4 x 4
+// 226 / 67 / 10.9; the groups of a launch in separate CTAs 242.
+constexpr int QXW = 4;  // 3-D: columns (warps) per CTA, of one plane
+constexpr int QW2 = 4;           // 2-D: columns (warps) per CTA
 
-// 16-byte async copy allocating in L1 as well (cp.async.ca).
-__device__ __forceinline__ void cp16ca(float4 *dst, const float *src, bool valid) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(dst);
-  const int n = valid ? 16 : 0;
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(src), "r"(n)
-               : "memory");
-}
+__device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 
-// One CTA's work: (bx, by) = (z chunk + x tile, y chunk) of the field that
-// `a` describes; `ring` is the CTA's dynamic shared memory.
-template <bool TWO_D, bool TRI, bool SNAP>
-__device__ __forceinline__ void march_body(const StepArgs &a, int bx, int by, float4 *ring) {
-  constexpr int NS = MARCH_NS, D = NS - 1;
+template <bool XT, bool TRI, bool SNAP>
+__device__ __forceinline__ void quad_update(const StepArgs &a, int slot, int ix, int y, int it,
+                                            bool swap) {
   const Geo &g = a.g;
-  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-  const int nth = blockDim.x;
-  const int G = a.ngroups;
-  const int spw = 32 / G;
-  const int gi = lane % G;
-  const int sl = lane / G;
-  const int xl = w / a.WPC;
-  const int zs = (w - xl * a.WPC) * spw + sl;
-  const int slot = (bx % a.nzc) * a.ZS + zs;
-  const int ix = TWO_D ? 0 : (bx / a.nzc) * a.KX + xl;
-  const bool valid = sl < spw && zs < a.ZS && slot < a.S && xl < a.KX && ix < g.nx;
   const int iz0 = 4 * slot - HZ;
-  const bool live = valid && slot >= 1 && iz0 < g.nz;
-  const float *A = a.cur[0];
-  float *B = a.nxt[0];
-#pragma unroll
-  for (int k = 1; k < MAXG; k++)
-    if (gi == k) {
-      A = a.cur[k];
-      B = a.nxt[k];
-    }
   const long long sx = g.sx, sy = g.sy;
-  const long long base = valid ? 4LL * slot + sx * (ix + g.hx) + sy * g.hy : 0;
-  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-
-  float wz[4];
-  bool lzm[4], keep[4];
-#pragma unroll
-  for (int e = 0; e < 4; e++) {
-    const int iz = iz0 + e;
-    wz[e] = (live && iz < g.nz) ? a.wz[iz] : 1.f;
-    lzm[e] = iz >= g.lz0 && iz < g.lz1;
-    keep[e] = iz < g.nz;
-  }
-  const float wx = (!TWO_D && live) ? a.wx[ix] : 1.f;
-  const bool lxm = TWO_D || (ix >= g.lx0 && ix < g.lx1);
-  const bool needL = valid && slot >= 1 && (sl == 0 || zs == 0);
-  const bool needR = valid && slot + 1 < a.S && (sl == spw - 1 || zs == a.ZS - 1);
+  // a plane of 2^32 floats would not fit the device: 32-bit strides and indices
+  const unsigned long long o = 4u * slot + (unsigned long long)(unsigned)sx * (unsigned)(ix + g.hx) +
+                               (unsigned long long)(unsigned)sy * (unsigned)(y + g.hy);
+  const float4 vv4 = ld4(a.vv + o);
+  const float4 wz4 = ld4(a.wz + iz0);
+  const float wz[4] = {wz4.x, wz4.y, wz4.z, wz4.w};
+  const float wx = XT ? a.wx[ix] : 1.f, wy = a.wy[y];
+  const f2 k1 = pk2(a.one, a.one);
+  // every cell of the float4 inside the Laplacian's region
+  const bool lxy = (!XT || (ix >= g.lx0 && ix < g.lx1)) && y >= g.ly0 && y < g.ly1;
+  const bool full = lxy && iz0 >= g.lz0 && iz0 + 3 < g.lz1;
   const int erz = a.rz - iz0;
-  const bool rec_zx = live && erz >= 0 && erz < 4 && ix >= a.rx0 && ix < a.rx0 + a.nrx;
-  const bool in_zx = ix >= a.nbx && ix < a.nbx + a.nx1;
-  const int nrec = a.nrx * a.nry;
-
-  const int y0 = by * a.ych;
-  const int y1 = min(g.ny, y0 + a.ych);
-  float4 *rA = ring, *rB = ring + NS * nth, *rV = ring + 2 * NS * nth;
-  // plane y's copies: A at y+2 (the queue's leading plane), B and vv at y
-  auto issue = [&](int y) {
-    if (y < y1) {
-      const int k = (y & (NS - 1)) * nth + t;
-      const long long o = base + sy * y;
-      cp16ca(rA + k, A + o + 2 * sy, valid);
-      cp16(rB + k, B + o, valid);
-      cp16(rV + k, a.vv + o, valid);
-    }
-    cp_commit();
-  };
-  float4 q0 = zero4, q1 = zero4, q2 = zero4, q3 = zero4;
-  if (valid) {
-    q0 = __ldg(reinterpret_cast<const float4 *>(A + base + sy * (y0 - 2)));
-    q1 = __ldg(reinterpret_cast<const float4 *>(A + base + sy * (y0 - 1)));
-    q2 = __ldg(reinterpret_cast<const float4 *>(A + base + sy * y0));
-    q3 = __ldg(reinterpret_cast<const float4 *>(A + base + sy * (y0 + 1)));
-  }
-#pragma unroll
-  for (int j = 0; j < D; j++) issue(y0 + j);
-  const unsigned full = 0xffffffffu;
-  for (int y = y0; y < y1; y++) {
-    issue(y + D);
-    cp_wait<D>();
-    const long long o = base + sy * y;
-    const int k = (y & (NS - 1)) * nth + t;
-    const float4 q4 = rA[k];
-    const float4 pv = rB[k];
-    const float4 vv4 = rV[k];
-    float4 xm1, xp1, xm2, xp2;
-    if (!TWO_D) {
-      xm1 = xp1 = xm2 = xp2 = zero4;
-      if (valid) {
-        xm1 = __ldg(reinterpret_cast<const float4 *>(A + o - sx));
-        xp1 = __ldg(reinterpret_cast<const float4 *>(A + o + sx));
-        xm2 = __ldg(reinterpret_cast<const float4 *>(A + o - 2 * sx));
-        xp2 = __ldg(reinterpret_cast<const float4 *>(A + o + 2 * sx));
-      }
-    }
-    float Lz = __shfl_up_sync(full, q2.z, G), Lw = __shfl_up_sync(full, q2.w, G);
-    float Rx = __shfl_down_sync(full, q2.x, G), Ry = __shfl_down_sync(full, q2.y, G);
-    if (needL) {
-      const float4 h = __ldg(reinterpret_cast<const float4 *>(A + o - 4));
-      Lz = h.z;
-      Lw = h.w;
-    }
-    if (needR) {
-      const float4 h = __ldg(reinterpret_cast<const float4 *>(A + o + 4));
-      Rx = h.x;
-      Ry = h.y;
-    }
-    const float wy = __ldg(a.wy + y);
-    const bool lyok = y >= g.ly0 && y < g.ly1;
-    const bool rec_here = rec_zx && y >= a.ry0 && y < a.ry0 + a.nry;
-    const int r_idx = rec_here ? (y - a.ry0) * a.nrx + (ix - a.rx0) : 0;
-    bool inj = false;
-    float dval = 0.f;
+  bool rec_here = false;  // this float4 holds a receiver
+  size_t r_off = 0;
+  int inj_g = -1;  // TRI: the group that injects here, and its sample
+  float dval = 0.f;
+  if ((unsigned)erz < 4u) {
+    const int rx = ix - a.rx0, ry = y - a.ry0;
+    rec_here = (unsigned)rx < (unsigned)a.nrx && (unsigned)ry < (unsigned)a.nry;
+    const int r_idx = ry * a.nrx + rx;
+    r_off = (size_t)it * (a.nrx * a.nry) + r_idx;
     if (TRI && rec_here) {
-      inj = a.gid == nullptr ? gi == 0 : a.gid[r_idx] == gi;
-      if (inj) dval = a.tri_dat[(size_t)a.it * nrec + r_idx];
+      inj_g = a.gid == nullptr ? 0 : a.gid[r_idx];
+      dval = a.tri_dat[r_off];
     }
-    bool src_plane = false;
-    if (!TRI)
-      for (int s = 0; s < a.ns; s++) src_plane |= (y >= a.sy[s] - 1 && y <= a.sy[s] + 1);
-    // prev = taper(u_{k-1} as stored); x1.0 outside the faces is exact
-    const f2 k1 = pk2(a.one, a.one);
-    float4 lap = lap_quad<!TWO_D>(a, k1, q2, q1, q3, q0, q4, xm1, xp1, xm2, xp2, Lz, Lw, Rx, Ry);
+  }
+  const bool in_xy = SNAP && ix >= a.nbx && ix < a.nbx + a.nx1 && y >= a.nby && y < a.nby + a.ny1;
+  float4 prod = make_float4(1.f, 1.f, 1.f, 1.f);
+  const int G = TRI ? a.ngroups : 1;
+#pragma unroll 1
+  for (int gi = 0; gi < G; gi++) {
+    const float *A = (swap ? a.nxt[gi] : a.cur[gi]) + o;
+    float *B = (swap ? const_cast<float *>(a.cur[gi]) : a.nxt[gi]) + o;
+    const float4 c = ld4(A), pv = ld4(B);
+    const float4 ym1 = ld4(A - sy), yp1 = ld4(A + sy);
+    const float4 ym2 = ld4(A - 2 * sy), yp2 = ld4(A + 2 * sy);
+    float4 xm1 = c, xp1 = c, xm2 = c, xp2 = c;
+    if (XT) {
+      xm1 = ld4(A - sx);
+      xp1 = ld4(A + sx);
+      xm2 = ld4(A - 2 * sx);
+      xp2 = ld4(A + 2 * sx);
+    }
+    const float2 zl = *reinterpret_cast<const float2 *>(A - 2);
+    const float2 zr = *reinterpret_cast<const float2 *>(A + 4);
+    float4 lap = lap_quad<XT>(a, k1, c, ym1, yp1, ym2, yp2, xm1, xp1, xm2, xp2, zl.x, zl.y, zr.x,
+                              zr.y);
+    if (!full) {
 #pragma unroll
-    for (int e = 0; e < 4; e++)
-      if (!(lzm[e] && lxm && lyok)) set_el(lap, e, 0.f);
-    float4 res = update_quad<!TWO_D>(k1, q2, pv, lap, vv4, wz, wx, wy);
+      for (int e = 0; e < 4; e++)
+        if (!(lxy && iz0 + e >= g.lz0 && iz0 + e < g.lz1)) set_el(lap, e, 0.f);
+    }
+    float4 res = update_quad<XT>(k1, c, pv, lap, vv4, wz, wx, wy);
+    if (TRI) {  // time reversal injects after the update and before the taper
+      if (inj_g == gi) {
 #pragma unroll
-    for (int e = 0; e < 4; e++) {
-      const float vve = el(vv4, e);
-      float v = el(res, e);
-      if (TRI) {
-        if (inj && e == erz) v = fadd(v, fmul(vve, dval));
-      } else if (src_plane) {
-        const int iz = iz0 + e;
-        for (int s = 0; s < a.ns; s++) {
-          const int dz = iz - a.sz[s], dxs = TWO_D ? 0 : ix - a.sx[s], dys = y - a.sy[s];
-          if (dz >= -1 && dz <= 1 && dxs >= -1 && dxs <= 1 && dys >= -1 && dys <= 1) {
-            const float den = (float)(abs(dxs) + abs(dys) + abs(dz) + 1);
-            v = fadd(v, fdiv(fmul(vve, a.rick[(size_t)s * a.nt + a.it]), den));
-          }
-        }
+        for (int e = 0; e < 4; e++)
+          if (e == erz) set_el(res, e, fadd(el(res, e), fmul(el(vv4, e), dval)));
       }
-      set_el(res, e, v);
-    }
-    res = taper_quad<!TWO_D>(res, wz, wx, wy);
-#pragma unroll
-    for (int e = 0; e < 4; e++)
-      if (!keep[e]) set_el(res, e, 0.f);
-    if (live) *reinterpret_cast<float4 *>(B + o) = res;
-    if (!TRI && rec_here && a.rec && gi == 0) a.rec[(size_t)a.it * nrec + r_idx] = el(res, erz);
-    if (SNAP) {
-      const bool interior = live && in_zx && y >= a.nby && y < a.nby + a.ny1;
-      if (a.wfd && gi == 0 && interior) {
+    } else if (!XT || ((unsigned)(iz0 - a.sbz) <= (unsigned)a.sbzn &&
+                       (unsigned)(y - a.sby) <= (unsigned)a.sbyn)) {
+      for (int s = 0; s < a.ns; s++) {
+        const int dys = y - a.sy[s], dxs = XT ? ix - a.sx[s] : 0, dz0 = iz0 - a.sz[s];
+        if ((unsigned)(dys + 1) > 2u || (unsigned)(dxs + 1) > 2u || dz0 < -4 || dz0 > 1) continue;
+        const float w = a.rick[(size_t)s * a.nt + it];
 #pragma unroll
         for (int e = 0; e < 4; e++) {
-          const int iz = iz0 + e;
-          if (iz >= a.nbz && iz < a.nbz + a.nz1)
-            a.wfd[((size_t)(y - a.nby) * a.nx1 + (ix - a.nbx)) * a.nz1 + (iz - a.nbz)] =
-                el(res, e);
-        }
-      }
-      if (TRI && a.img != nullptr) {
-        // prod_g u_g^2 in group order; the groups of a slot sit in lanes sl*G + gg
-        float4 prod = make_float4(1.f, 1.f, 1.f, 1.f);
-        for (int gg = 0; gg < G; gg++) {
-          const int src = sl * G + gg;
-          float4 u;
-          u.x = __shfl_sync(full, res.x, src);
-          u.y = __shfl_sync(full, res.y, src);
-          u.z = __shfl_sync(full, res.z, src);
-          u.w = __shfl_sync(full, res.w, src);
-          prod.x = fmul(fmul(prod.x, u.x), u.x);
-          prod.y = fmul(fmul(prod.y, u.y), u.y);
-          prod.z = fmul(fmul(prod.z, u.z), u.z);
-          prod.w = fmul(fmul(prod.w, u.w), u.w);
-        }
-        if (gi == 0 && interior) {
-          float4 im = *reinterpret_cast<const float4 *>(a.img + o);
-#pragma unroll
-          for (int e = 0; e < 4; e++) {
-            const int iz = iz0 + e;
-            if (iz >= a.nbz && iz < a.nbz + a.nz1) set_el(im, e, fadd(el(im, e), el(prod, e)));
+          const int dz = dz0 + e;
+          if (dz >= -1 && dz <= 1) {
+            const float den = (float)(abs(dxs) + abs(dys) + abs(dz) + 1);
+            set_el(res, e, fadd(el(res, e), fdiv(fmul(el(vv4, e), w), den)));
           }
-          *reinterpret_cast<float4 *>(a.img + o) = im;
         }
       }
     }
-    q0 = q1;
-    q1 = q2;
-    q2 = q3;
-    q3 = q4;
+    // cells beyond nz stay zero: every operand is zero there
+    res = taper_quad<XT>(res, wz, wx, wy);
+    *reinterpret_cast<float4 *>(B) = res;
+    if (!TRI && rec_here && a.rec) a.rec[r_off] = el(res, erz);
+    if (SNAP && a.wfd && gi == 0 && in_xy) {
+      float *w = a.wfd + ((size_t)(y - a.nby) * a.nx1 + (ix - a.nbx)) * a.nz1 + (iz0 - a.nbz);
+#pragma unroll
+      for (int e = 0; e < 4; e++)
+        if (iz0 + e >= a.nbz && iz0 + e < a.nbz + a.nz1) w[e] = el(res, e);
+    }
+    if (SNAP && TRI) {
+      prod.x = fmul(fmul(prod.x, res.x), res.x);
+      prod.y = fmul(fmul(prod.y, res.y), res.y);
+      prod.z = fmul(fmul(prod.z, res.z), res.z);
+      prod.w = fmul(fmul(prod.w, res.w), res.w);
+    }
   }
-  cp_wait_all();
+  if (SNAP && TRI && a.img && in_xy && iz0 + 3 >= a.nbz && iz0 < a.nbz + a.nz1) {
+    // the demos' image (test_third_tri.py:71-77): img += prod_g u_g^2
+    float4 im = ld4(a.img + o);
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+      if (iz0 + e >= a.nbz && iz0 + e < a.nbz + a.nz1) set_el(im, e, fadd(el(im, e), el(prod, e)));
+    *reinterpret_cast<float4 *>(a.img + o) = im;
+  }
 }
 
-template <bool TWO_D, bool TRI, bool SNAP>
-__global__ void __launch_bounds__(MARCH_MAXT) march_kernel(const StepArgs a) {
-  extern __shared__ float4 ring[];
-  march_body<TWO_D, TRI, SNAP>(a, blockIdx.x, blockIdx.y, ring);
+// lane -> (column group, slot): lanes are numbered nq * group + slot - 1, so
+// none is idle whatever the depth (a warp may hold the end of one column and
+// the start of the next group's)
+__device__ __forceinline__ int quad_slot(const StepArgs &a, unsigned block, int &group) {
+  const unsigned item = block * 32 + (threadIdx.x & 31);
+  group = fast_div(item, a.nq);
+  return (int)item - group * a.nq.d + 1;
+}
+
+// Counts of the warps' groups by taper class, kept only when a.stats is set
+// (one warp-plane each): 0 no taper and no mask, 1 y taper only, 2 z / x taper
+// only, 3 anything else (both, masks, sources, injection).  [0..3] TRI,
+// [4..7] forward.
+template <bool TRI>
+__device__ __forceinline__ void quad_stats(const StepArgs &a, bool live, int slot, int ix, int y) {
+  const Geo &g = a.g;
+  const unsigned full = 0xffffffffu;
+  const int iz0 = 4 * slot - HZ;
+  bool tz = false, tx = false, ty = false, special = false;
+  if (live) {
+    const float4 w = ld4(a.wz + iz0);
+    tz = w.x != 1.f || w.y != 1.f || w.z != 1.f || w.w != 1.f;
+    tx = a.wx[ix] != 1.f;
+    ty = a.wy[y] != 1.f;
+    special = !(iz0 >= g.lz0 && iz0 + 3 < g.lz1 && ix >= g.lx0 && ix < g.lx1 && y >= g.ly0 &&
+                y < g.ly1);
+    if (TRI) special |= a.rz >= iz0 && a.rz < iz0 + 4 && ix >= a.rx0 && ix < a.rx0 + a.nrx &&
+                        y >= a.ry0 && y < a.ry0 + a.nry;
+    else
+      for (int s = 0; s < a.ns; s++) special |= abs(y - a.sy[s]) <= 1;
+  }
+  const bool any_live = __any_sync(full, live), zx = __any_sync(full, tz || tx);
+  const bool edge = __any_sync(full, tz && tx), yy = __any_sync(full, ty);
+  const bool sp = __any_sync(full, special);
+  if ((threadIdx.x & 31) == 0 && any_live) {
+    const int cls = sp || edge || (zx && yy) ? 3 : (zx ? 2 : (yy ? 1 : 0));
+    atomicAdd(a.stats + (TRI ? cls : 4 + cls), (unsigned long long)(TRI ? a.ngroups : 1));
+  }
+}
+
+// 3-D: QXW columns of one plane per CTA
+template <bool TRI, bool SNAP>
+__global__ void __launch_bounds__(32 * QXW, 6)
+    quad3_kernel(const __grid_constant__ StepArgs a) {
+  int group;
+  const int slot = quad_slot(a, blockIdx.x, group);
+  const int ix = group * QXW + (threadIdx.x >> 5);
+  pdl_wait();
+  pdl_launch();
+  // a launch has at most 65535 block rows: further planes along blockIdx.z
+  const int y = zigzag(a.it & a.zig, blockIdx.z * gridDim.y + blockIdx.y, gridDim.y * gridDim.z);
+  const bool live = ix < a.g.nx && y < a.g.ny;
+  if (a.stats != nullptr) quad_stats<TRI>(a, live, slot, ix, y);
+  if (live) quad_update<true, TRI, SNAP>(a, slot, ix, y, a.it, false);
+}
+
+// 2-D: QW2 columns of the kernel's y (the model's x) per CTA
+template <bool TRI, bool SNAP>
+__global__ void __launch_bounds__(32 * QW2) quad2_kernel(const __grid_constant__ StepArgs a) {
+  int group;
+  const int slot = quad_slot(a, zigzag(a.it & a.zig, blockIdx.x, gridDim.x), group);
+  const int y = group * QW2 + (threadIdx.x >> 5);
+  pdl_wait();
+  pdl_launch();
+  if (y < a.g.ny) quad_update<false, TRI, SNAP>(a, slot, 0, y, a.it, false);
 }
 
 // Cluster-resident 2-D propagation for grids that fit in the distributed
@@ -420,7 +394,7 @@ __global__ void __launch_bounds__(MARCH_MAXT) march_kernel(const StepArgs a) {
 // columns also into the neighbours' halo columns (distributed shared memory
 // stores), and ends with one cluster barrier; the next step reads the halos
 // locally.  Domain edges keep zero halos, as the global layout does.  The
-// arithmetic per cell is march_body's, term by term, so results are
+// arithmetic per cell is quad_update's, term by term, so results are
 // bit-identical to the step-per-launch path.
 constexpr int RES_NTH = 512;   // threads per CTA
 constexpr int RES_MAXIPT = 8;  // items (float4 of z cells) per thread, at most
@@ -642,30 +616,39 @@ __global__ void __launch_bounds__(RES_NTH) resident_kernel(const __grid_constant
 
 // Batched 2-D forward modelling of shots of uneven size and length: one
 // launch per time step covers the tiles of every shot still running.  Item
-// i = (shot, tile) with tile = z chunk + nzc * y chunk; items are ordered by
-// decreasing shot length so that the launch at step `it` takes a prefix.
-// The shot's arguments are copied into shared memory; A and B of a shot swap
-// roles with the parity of the step.
-__global__ void __launch_bounds__(MARCH_MAXT) batch_kernel(const StepArgs *args, const int2 *items,
-                                                           int it) {
-  extern __shared__ float4 ring[];
-  __shared__ StepArgs sa;
-  const int2 item = items[blockIdx.x];
-  const int *src = reinterpret_cast<const int *>(args + item.x);
-  int *dst = reinterpret_cast<int *>(&sa);
-  for (int i = threadIdx.x; i < (int)(sizeof(StepArgs) / sizeof(int)); i += blockDim.x)
-    dst[i] = src[i];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    sa.it = it;
-    if (it & 1) {
-      float *t = sa.nxt[0];
-      sa.nxt[0] = const_cast<float *>(sa.cur[0]);
-      sa.cur[0] = t;
-    }
+// i = (shot, block of the shot's lanes); items are ordered by decreasing shot
+// length so that the launch at step `it` takes a prefix.  A and B of a shot
+// swap roles with the parity of the step.  The shots' arguments sit in
+// constant memory, read like kernel parameters, when there are at most
+// BATCH_TAB of them (TAB); otherwise each CTA copies its shot's into shared
+// memory first.  The table is written and read under the device's workspace
+// lock only.
+constexpr int BATCH_TAB = 96;
+__constant__ char batch_tab[BATCH_TAB * sizeof(StepArgs)];
+
+template <bool TAB>
+__global__ void __launch_bounds__(32 * QW2) batch_kernel(const StepArgs *args, const int2 *items,
+                                                         int it, int zig) {
+  const int2 item = items[zigzag(it & zig, blockIdx.x, gridDim.x)];
+  int group;
+  if constexpr (TAB) {
+    const StepArgs &sa = reinterpret_cast<const StepArgs *>(batch_tab)[item.x];
+    const int slot = quad_slot(sa, item.y, group), y = group * QW2 + (threadIdx.x >> 5);
+    pdl_wait();
+    pdl_launch();
+    if (y < sa.g.ny) quad_update<false, false, false>(sa, slot, 0, y, it, (it & 1) != 0);
+  } else {
+    __shared__ StepArgs sa;
+    const int *src = reinterpret_cast<const int *>(args + item.x);
+    int *dst = reinterpret_cast<int *>(&sa);
+    for (int i = threadIdx.x; i < (int)(sizeof(StepArgs) / sizeof(int)); i += 32 * QW2)
+      dst[i] = src[i];
+    __syncthreads();
+    const int slot = quad_slot(sa, item.y, group), y = group * QW2 + (threadIdx.x >> 5);
+    pdl_wait();
+    pdl_launch();
+    if (y < sa.g.ny) quad_update<false, false, false>(sa, slot, 0, y, it, (it & 1) != 0);
   }
-  __syncthreads();
-  march_body<true, false, false>(sa, item.y % sa.nzc, item.y / sa.nzc, ring);
 }
 
 // Warp-tile kernels (3-D): each warp owns an 8-slot x 4*NC-column patch of
@@ -1447,28 +1430,38 @@ struct Plan {
   dim3 grid;
   size_t smem;
   void *fn, *fn_snap;  // plain steps / snapshot and imaging steps
-  bool tile;           // warp-tile kernel: TRI images by image_kernel
+  bool quad;           // quad kernel; otherwise a warp-tile kernel (TRI images by image_kernel)
   bool tma;            // warp-tile kernel with the TMA ring (takes TileMaps)
   int nc;              // warp-tile kernel: columns per lane
   int threads;
-  int S, ZS, KX, nzc, WPC, WZ, WX;
+  FastDiv nq;
+  int S, nzc, WZ, WX;
 };
 
-template <bool TWO_D, bool TRI, bool SNAP>
-static void *march_ptr() {
-  void *f = (void *)march_kernel<TWO_D, TRI, SNAP>;
-  static bool once = [f] {
-    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         3 * MARCH_NS * MARCH_MAXT * (int)sizeof(float4));
-    return true;
-  }();
-  (void)once;
-  return f;
+template <bool TWO_D>
+static void *quad_fn(bool tri, bool snap) {
+  if (TWO_D) {
+    if (tri) return snap ? (void *)quad2_kernel<true, true> : (void *)quad2_kernel<true, false>;
+    return snap ? (void *)quad2_kernel<false, true> : (void *)quad2_kernel<false, false>;
+  }
+  if (tri) return snap ? (void *)quad3_kernel<true, true> : (void *)quad3_kernel<true, false>;
+  return snap ? (void *)quad3_kernel<false, true> : (void *)quad3_kernel<false, false>;
 }
 
-static void *march_fn(bool tri, bool snap) {  // 2-D runs
-  if (tri) return snap ? march_ptr<true, true, true>() : march_ptr<true, true, false>();
-  return snap ? march_ptr<true, false, true>() : march_ptr<true, false, false>();
+static void plan_quad(bool tri, int G, Plan &p) {
+  const Geo &g = p.g;
+  const bool two_d = p.dim == 2;
+  p.quad = true;
+  p.fn = two_d ? quad_fn<true>(tri, false) : quad_fn<false>(tri, false);
+  p.fn_snap = two_d ? quad_fn<true>(tri, true) : quad_fn<false>(tri, true);
+  const long long lanes = (long long)p.nq.d * (two_d ? ceil_div(g.ny, QW2) : ceil_div(g.nx, QXW));
+  p.grid = dim3((unsigned)ceil_div(lanes, 32), two_d ? 1u : (unsigned)std::min(g.ny, 65535),
+                two_d ? 1u : (unsigned)ceil_div(g.ny, 65535));
+  p.threads = 32 * (two_d ? QW2 : QXW);
+  p.smem = 0;
+  if (getenv("PW_AFD_VERBOSE"))
+    fprintf(stderr, "afd quad plan: G=%d nq=%d threads=%d grid=%ux%u\n", G, p.nq.d, p.threads,
+            p.grid.x, p.grid.y);
 }
 
 // Tile override for measurements: PW_AFD_TILE_G<G>="a,b" fixes the first two
@@ -1478,81 +1471,6 @@ static void tile_override(int G, int &fa, int &fb) {
   char name[32];
   snprintf(name, sizeof name, "PW_AFD_TILE_G%d", G);
   if (const char *e = getenv(name)) sscanf(e, "%d,%d", &fa, &fb);
-}
-
-// Tile of the march kernel: WPC warps per z chunk of ZS = WPC * (32/G) slots,
-// KX columns per CTA, ych planes per CTA.  Score = useful thread-planes /
-// thread-plane capacity spent (idle lanes, dead slots, partial waves, the
-// 2-plane prologue of each y chunk), times a latency factor below 24 resident
-// warps per SM and a penalty for x-neighbour loads served by other CTAs.
-static int plan_march(bool tri, int G, int nsm, Plan &p) {
-  const Geo &g = p.g;
-  const bool two_d = p.dim == 2;
-  void *fn = march_fn(tri, false);
-  const int S = g.lz / 4;
-  const int spw = 32 / G;
-  const int live_slots = ceil_div(g.nz, 4);
-  const double useful = (double)G * live_slots * g.nx * g.ny;
-  int fw, fk;
-  tile_override(G, fw, fk);
-  double best = -1;
-  int bw = 0, bk = 0, by = 0;
-  for (int WPC = 1; WPC <= ceil_div(S, spw); WPC++) {
-    if (fw && WPC != fw) continue;
-    const int ZS = WPC * spw;
-    const int nzc = ceil_div(S, ZS);
-    if (WPC > 1 && ceil_div(S, (WPC - 1) * spw) == nzc) continue;  // same chunks, fewer lanes
-    for (int KX = 1; KX <= (two_d ? 1 : 64); KX++) {
-      const int threads = 32 * WPC * KX;
-      if (threads > MARCH_MAXT) break;
-      if (fk && KX != fk) continue;
-      const size_t smem = (size_t)3 * MARCH_NS * threads * sizeof(float4);
-      int occ = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, smem) != cudaSuccess) {
-        cudaGetLastError();
-        occ = 0;
-      }
-      if (occ <= 0) continue;
-      const long long slots = (long long)nsm * occ;
-      const long long tiles = (long long)nzc * ceil_div(g.nx, KX);
-      const double warps = (double)occ * threads / 32;
-      const double lat = std::min(1.0, warps / 24.0);
-      const double outside = two_d ? 0.0 : (KX == 1 ? 1.0 : 6.0 / (4.0 * KX));
-      const double xh = 1.0 / (1.0 + 0.3 * outside);
-      for (int ych = std::max(4, ceil_div(g.ny, 65535)); ych <= g.ny + 3; ych++) {
-        const int yc = std::min(ych, g.ny);
-        const long long ctas = tiles * ceil_div(g.ny, yc);
-        const long long waves = (ctas + slots - 1) / slots;
-        const double cap = (double)waves * slots * threads * (yc + 2);
-        const double score = useful / cap * lat * xh;
-        if (score > best + 1e-9) {
-          best = score;
-          bw = WPC;
-          bk = KX;
-          by = yc;
-        }
-        if (yc == g.ny) break;
-      }
-    }
-  }
-  PW_CHECK(best > 0, PW_ERR_SHAPE, "no launchable tile for the step kernel");
-  p.fn = fn;
-  p.fn_snap = march_fn(tri, true);
-  p.S = S;
-  p.WPC = bw;
-  p.ZS = bw * spw;
-  p.nzc = ceil_div(S, p.ZS);
-  p.KX = bk;
-  p.ych = by;
-  p.threads = 32 * bw * bk;
-  p.smem = (size_t)3 * MARCH_NS * p.threads * sizeof(float4);
-  p.grid = dim3((unsigned)(p.nzc * ceil_div(g.nx, bk)), (unsigned)ceil_div(g.ny, by), 1);
-  if (getenv("PW_AFD_VERBOSE"))
-    fprintf(stderr,
-            "afd march plan: G=%d S=%d nzc=%d ZS=%d WPC=%d KX=%d ych=%d threads=%d grid=%ux%u "
-            "score=%.3f\n",
-            G, S, p.nzc, p.ZS, bw, bk, by, p.threads, p.grid.x, p.grid.y, best);
-  return PW_OK;
 }
 
 // split B / vv ring of the cp.async kernel (3 slots of B and vv beside the
@@ -1679,7 +1597,6 @@ static int plan_tile(bool tri, int G, int nsm, bool tma, Plan &p) {
   PW_CHECK(best > 0, PW_ERR_SHAPE, "no launchable tile for the step kernel");
   p.fn = tile_fn(tri, false, tma, bnc);
   p.fn_snap = tile_fn(tri, true, tma, bnc);
-  p.tile = true;
   p.tma = tma;
   p.nc = bnc;
   p.S = S;
@@ -1698,6 +1615,13 @@ static int plan_tile(bool tri, int G, int nsm, bool tma, Plan &p) {
             G, S, p.nzc, bz, bx, bnc, by, p.threads, p.grid.x, p.grid.y, best,
             tma ? "tma" : (tile_split(bnc) ? "cp.async+split" : "cp.async"));
   return PW_OK;
+}
+
+// A warp-tile variant is asked for.
+static bool tile_selected(int G) {
+  int a, b;
+  tile_override(G, a, b);
+  return a > 0 || getenv("PW_AFD_TMA") || getenv("PW_AFD_SPLIT") || getenv("PW_AFD_NC");
 }
 
 static int make_plan(const pw_afd_args *a, bool tri, int G, Plan &p, bool allow_tma = true) {
@@ -1744,10 +1668,12 @@ static int make_plan(const pw_afd_args *a, bool tri, int G, Plan &p, bool allow_
   int dev = 0, nsm = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  p.S = p.ZS = p.KX = p.nzc = p.WPC = p.WZ = p.WX = 0;
-  p.tile = p.tma = false;
+  p.S = p.nzc = p.WZ = p.WX = 0;
+  p.quad = p.tma = false;
   p.nc = 1;
-  if (two_d) PW_TRY(plan_march(tri, G, nsm, p));  // 2-D: no x neighbours to stage
+  p.ych = 0;
+  p.nq = make_fast_div(ceil_div(g.nz, 4));
+  if (two_d || !tile_selected(G)) plan_quad(tri, G, p);
   else PW_TRY(plan_tile(tri, G, nsm, allow_tma && tile_use_tma(), p));
   return PW_OK;
 }
@@ -1933,6 +1859,37 @@ static int tile_maps(const Geo &g, int G, int nc, float *const *buf0, float *con
   return PW_OK;
 }
 
+// Ranges of the float4s and planes that hold a cell of a source's spread.
+static void source_box(StepArgs &s) {
+  int z0 = 1 << 30, z1 = -(1 << 30), y0 = z0, y1 = z1;
+  for (int i = 0; i < s.ns; i++) {
+    z0 = std::min(z0, s.sz[i] - 4);
+    z1 = std::max(z1, s.sz[i] + 1);
+    y0 = std::min(y0, s.sy[i] - 1);
+    y1 = std::max(y1, s.sy[i] + 1);
+  }
+  const bool any = s.ns > 0;
+  s.sbz = any ? z0 : 1 << 30;  // no iz0 or y is as large
+  s.sbzn = any ? z1 - z0 : 0;
+  s.sby = any ? y0 : 1 << 30;
+  s.sbyn = any ? y1 - y0 : 0;
+}
+
+// One step; the quad kernels may overlap their start with the step before.
+static cudaError_t launch_step(void *fn, const Plan &p, void **args, cudaStream_t st) {
+  if (!p.quad) return cudaLaunchKernel(fn, p.grid, dim3(p.threads), args, p.smem, st);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = p.grid;
+  cfg.blockDim = dim3(p.threads);
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
 static int run(const pw_afd_args *a, int G, const int *group, const float *vel, const float *src,
                const float *wavelet, float *dat, float *wfd, float *img_out, int normalize,
                cudaStream_t st) {
@@ -2009,6 +1966,7 @@ static int run(const pw_afd_args *a, int G, const int *group, const float *vel, 
     w[ib] = (float)exp(-a->ct * a->ct * (p.nb - 1 - ib) * (p.nb - 1 - ib));
   std::vector<float> wz, wx, wy;
   taper_axis(g.nz, p.nz2, p.nb, w, wz);
+  wz.resize(round_up(g.nz, 4), 1.f);  // read four at a time
   if (two_d) {
     wx.assign(1, 1.f);
     taper_axis(g.ny, p.nx2, p.nb, w, wy);
@@ -2040,7 +1998,7 @@ static int run(const pw_afd_args *a, int G, const int *group, const float *vel, 
   const size_t o_wfd = cv.add(wfd && host ? (size_t)ntsnap * nvel * 4 : 0);
   const size_t o_mx = cv.add(16);
   // PW_AFD_VERBOSE: also count which paths the 3-D step kernels took
-  const bool want_stats = p.tile && getenv("PW_AFD_VERBOSE") != nullptr;
+  const bool want_stats = !two_d && getenv("PW_AFD_VERBOSE") != nullptr;
   const size_t o_stats = cv.add(want_stats ? 8 * sizeof(unsigned long long) : 0);
   const size_t o_err = cv.add(p.tma ? 16 : 0);
 
@@ -2112,11 +2070,10 @@ static int run(const pw_afd_args *a, int G, const int *group, const float *vel, 
   s.g = g;
   s.ych = p.ych;
   s.ngroups = G;
+  s.zig = zigzag_pays((size_t)(2 * G + 1) * nfield * 4);
   s.S = p.S;
-  s.ZS = p.ZS;
-  s.KX = p.KX;
   s.nzc = p.nzc;
-  s.WPC = p.WPC;
+  s.nq = p.nq;
   s.WZ = p.WZ;
   s.WX = p.WX;
   {
@@ -2149,6 +2106,7 @@ static int run(const pw_afd_args *a, int G, const int *group, const float *vel, 
     s.sx[i] = ksx[i];
     s.sy[i] = ksy[i];
   }
+  source_box(s);
   s.rick = d_rick;
   s.rz = p.nb + a->gz;
   if (two_d) {
@@ -2167,7 +2125,6 @@ static int run(const pw_afd_args *a, int G, const int *group, const float *vel, 
   if (p.tma) PW_TRY(tile_maps(g, G, p.nc, A, B, vv, maps));
   float *wfd_dev = wfd ? (host ? at<float>(base, o_wfd) : wfd) : nullptr;
   void *fn = p.fn;
-  const int threads = p.threads;
   ImgArgs ia{};
   ia.g = g;
   ia.G = G;
@@ -2220,11 +2177,11 @@ static int run(const pw_afd_args *a, int G, const int *group, const float *vel, 
     const bool snap = a->jsnap > 0 && it % a->jsnap == 0;
     s.wfd = (snap && wfd_dev) ? wfd_dev + (size_t)(it / a->jsnap) * nvel : nullptr;
     const bool img_step = snap && img;
-    s.img = (img_step && !p.tile) ? img : nullptr;
+    s.img = (img_step && p.quad) ? img : nullptr;
     void *args[] = {(void *)&s, (void *)&maps[k & 1]};
     void *f = (s.wfd || s.img) ? p.fn_snap : fn;
-    PW_CUDA(cudaLaunchKernel(f, p.grid, dim3(threads), args, p.smem, st));
-    if (img_step && p.tile) {
+    PW_CUDA(launch_step(f, p, args, st));
+    if (img_step && !p.quad) {
       for (int i = 0; i < G; i++) ia.u[i] = B[i];
       image_kernel<<<1184, 256, 0, st>>>(ia);
       img_launches++;
@@ -2336,6 +2293,7 @@ static int batch_setup(const pw_afd_args *a, const float *src, const float *wave
   for (int ib = 0; ib < p.nb; ib++)
     w[ib] = (float)exp(-a->ct * a->ct * (p.nb - 1 - ib) * (p.nb - 1 - ib));
   taper_axis(g.nz, p.nz2, p.nb, w, b.wz);
+  b.wz.resize(round_up(g.nz, 4), 1.f);  // read four at a time
   taper_axis(g.ny, p.nx2, p.nb, w, b.wy);
   b.nvel = (size_t)p.nz1 * p.nx1;
   b.nrec = (size_t)p.nx1;
@@ -2382,6 +2340,7 @@ static void batch_args(const pw_afd_args *a, const BatchShot &b, char *base, Ste
     s.sx[i] = 0;
     s.sy[i] = b.ksy[i];
   }
+  source_box(s);
   s.rick = at<float>(base, b.o_rick);
   s.rz = p.nb + a->gz;
   s.rx0 = 0;
@@ -2395,32 +2354,7 @@ static void batch_args(const pw_afd_args *a, const BatchShot &b, char *base, Ste
   s.nz1 = p.knz1;
   s.nx1 = p.knx1;
   s.ny1 = p.kny1;
-  s.S = p.g.lz / 4;
-  s.KX = 1;
-}
-
-// A batch tile: WPC warps per z chunk (ZS = 32 * WPC slots), ych planes.
-struct BatchTile {
-  int wpc, ych;
-};
-
-// Sets the tile fields of every shot and builds the (shot, tile) items in
-// decreasing shot length; cum[k] = items of the k longest shots.
-static void batch_items(const BatchTile &t, const std::vector<int> &order,
-                        std::vector<StepArgs> &args, std::vector<int2> &items,
-                        std::vector<int> &cum) {
-  items.clear();
-  cum.assign(1, 0);
-  for (int k : order) {
-    StepArgs &s = args[k];
-    s.WPC = t.wpc;
-    s.ZS = 32 * t.wpc;
-    s.nzc = ceil_div(s.S, s.ZS);
-    s.ych = std::min(t.ych, s.g.ny);
-    const int tiles = s.nzc * ceil_div(s.g.ny, s.ych);
-    for (int i = 0; i < tiles; i++) items.push_back(make_int2(k, i));
-    cum.push_back((int)items.size());
-  }
+  s.nq = p.nq;
 }
 
 static int run_batch(int nshot, const pw_afd_args *args, const float *const *vel,
@@ -2445,19 +2379,10 @@ static int run_batch(int nshot, const pw_afd_args *args, const float *const *vel
     ntmax = std::max(ntmax, args[k].nt);
   }
   const size_t o_args = cv.add((size_t)nshot * sizeof(StepArgs));
-  size_t max_items = 0;
-  const BatchTile cands[] = {{1, 16}, {1, 32}, {2, 32}, {2, 64}, {4, 32}, {4, 64}};
-  const int ncand = (int)(sizeof cands / sizeof cands[0]);
-  for (const BatchTile &t : cands) {
-    size_t n = 0;
-    for (int k = 0; k < nshot; k++) {
-      const Geo &g = shots[k].p.g;
-      n += (size_t)ceil_div(g.lz / 4, 32 * t.wpc) * ceil_div(g.ny, std::min(t.ych, g.ny));
-    }
-    max_items = std::max(max_items, n);
-  }
-  PW_CHECK(max_items < (1u << 31), PW_ERR_SHAPE, "too many tiles");
-  const size_t o_items = cv.add(max_items * sizeof(int2));
+  size_t nitems = 0;
+  for (const BatchShot &b : shots) nitems += b.p.grid.x;
+  PW_CHECK(nitems < (1u << 31), PW_ERR_SHAPE, "too many tiles");
+  const size_t o_items = cv.add(nitems * sizeof(int2));
 
   Workspace &ws = Workspace::for_current_device();
   std::lock_guard<std::mutex> lock(ws.mutex());
@@ -2502,85 +2427,44 @@ static int run_batch(int nshot, const pw_afd_args *args, const float *const *vel
   for (int k = 0; k < nshot; k++) nt_sorted[k] = args[order[k]].nt;
   StepArgs *d_args = at<StepArgs>(base, o_args);
   int2 *d_items = at<int2>(base, o_items);
+  // (shot, block) items, longest shots first; cum[k] = items of the k longest
   std::vector<int2> items;
-  std::vector<int> cum;
-  {
-    static bool attr = [] {
-      cudaFuncSetAttribute((const void *)batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           3 * MARCH_NS * MARCH_MAXT * (int)sizeof(float4));
-      return true;
-    }();
-    (void)attr;
+  std::vector<int> cum(1, 0);
+  items.reserve(nitems);
+  for (int k : order) {
+    for (int i = 0; i < (int)shots[k].p.grid.x; i++) items.push_back(make_int2(k, i));
+    cum.push_back((int)items.size());
   }
-  auto use_tile = [&](const BatchTile &t) -> int {
-    batch_items(t, order, sargs, items, cum);
+  const bool tab = nshot <= BATCH_TAB;
+  if (tab)
+    PW_CUDA(cudaMemcpyToSymbolAsync(batch_tab, sargs.data(), sargs.size() * sizeof(StepArgs), 0,
+                                    cudaMemcpyHostToDevice, st));
+  else
     PW_CUDA(cudaMemcpyAsync(d_args, sargs.data(), sargs.size() * sizeof(StepArgs),
                             cudaMemcpyHostToDevice, st));
-    PW_CUDA(cudaMemcpyAsync(d_items, items.data(), items.size() * sizeof(int2),
-                            cudaMemcpyHostToDevice, st));
-    PW_CUDA(cudaStreamSynchronize(st));  // host vectors are reused
-    return PW_OK;
-  };
-  int tile_threads = 32;
-  size_t tile_smem = 0;
+  PW_CUDA(cudaMemcpyAsync(d_items, items.data(), items.size() * sizeof(int2),
+                          cudaMemcpyHostToDevice, st));
+  PW_CUDA(cudaStreamSynchronize(st));  // host vectors
+  if (getenv("PW_AFD_VERBOSE"))
+    fprintf(stderr, "afd batch: %d shots, %zu items\n", nshot, items.size());
   // running shots at step it: the first n with nt_sorted[n - 1] > it
   int running = nshot;
+  size_t fbytes = 0;
+  for (const BatchShot &b : shots) fbytes += 3 * b.nfield * 4;
+  const int zig = zigzag_pays(fbytes);
   auto step = [&](int it) -> int {
     while (running > 0 && nt_sorted[running - 1] <= it) running--;
     const int n = cum[running];
     if (n == 0) return PW_OK;
-    batch_kernel<<<n, tile_threads, tile_smem, st>>>(d_args, d_items, it);
-    PW_CUDA(cudaGetLastError());
+    PW_CUDA(launch_pdl(tab ? batch_kernel<true> : batch_kernel<false>, dim3(n), dim3(32 * QW2), 0,
+                       st, (const StepArgs *)d_args, (const int2 *)d_items, it, zig));
     return PW_OK;
   };
-
-  // Online tile tuning on the first real steps: every tile computes the same
-  // values, so each candidate simply takes two steps, timed by events; the
-  // fastest runs the rest.  Short runs keep the first candidate.
-  const int tune_steps = 2;
-  int best = 0;
   int it = 0;
   LoopTimer timer(st);
   timer.start();
   long long launches = 0;
-  if (ntmax >= 8 * ncand * tune_steps) {
-    float best_ms = 1e30f;
-    cudaEvent_t e0, e1;
-    PW_CUDA(cudaEventCreate(&e0));
-    PW_CUDA(cudaEventCreate(&e1));
-    int rc = PW_OK;
-    for (int c = 0; c < ncand && rc == PW_OK; c++) {
-      rc = use_tile(cands[c]);
-      if (rc != PW_OK) break;
-      tile_threads = 32 * cands[c].wpc;
-      tile_smem = (size_t)3 * MARCH_NS * tile_threads * sizeof(float4);
-      cudaEventRecord(e0, st);
-      for (int j = 0; j < tune_steps && rc == PW_OK; j++, it++, launches++) rc = step(it);
-      cudaEventRecord(e1, st);
-      cudaEventSynchronize(e1);
-      float ms = 0.f;
-      cudaEventElapsedTime(&ms, e0, e1);
-      // per cell-update (later steps may have fewer running shots)
-      double cells = 0;
-      for (int k = 0; k < nshot; k++)
-        if (args[k].nt > it - tune_steps) cells += (double)shots[k].p.g.nz * shots[k].p.g.ny;
-      const float norm = cells > 0 ? (float)(ms / cells) : ms;
-      if (norm < best_ms) {
-        best_ms = norm;
-        best = c;
-      }
-    }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    PW_TRY(rc);
-  }
-  PW_TRY(use_tile(cands[best]));
-  tile_threads = 32 * cands[best].wpc;
-  tile_smem = (size_t)3 * MARCH_NS * tile_threads * sizeof(float4);
-  if (getenv("PW_AFD_VERBOSE"))
-    fprintf(stderr, "afd batch: %d shots, tile wpc=%d ych=%d, %zu items\n", nshot,
-            cands[best].wpc, cands[best].ych, items.size());
-  // the remaining steps replay as one CUDA graph (direct launches on the
+  // the steps replay as one CUDA graph (direct launches on the
   // legacy default stream, which cannot be captured)
   bool graphed = false;
   if (st != nullptr && it < ntmax) {
@@ -2708,7 +2592,8 @@ static int run_noalloc(const pw_afd_args *a, const float *vel, const float *src,
   const size_t o_A = cv.add(nfield * 4);
   const size_t o_B = cv.add(nfield * 4);
   const size_t o_w = cv.add((size_t)p.nb * 4);
-  const size_t o_t = cv.add((size_t)(g.nz + g.nx + g.ny) * 4);
+  const int nzt = (int)round_up(g.nz, 4);  // the z table is read four at a time
+  const size_t o_t = cv.add((size_t)(nzt + g.nx + g.ny) * 4);
   const size_t o_rec = cv.add(dat ? (size_t)nt * nrec * 4 : 0);
   const size_t o_mx = cv.add(16);
   const size_t need = cv.total();
@@ -2739,7 +2624,7 @@ static int run_noalloc(const pw_afd_args *a, const float *vel, const float *src,
   float *vv = at<float>(base, o_vv);
   float *A = at<float>(base, o_A), *B = at<float>(base, o_B);
   float *d_w = at<float>(base, o_w);
-  float *d_wz = at<float>(base, o_t), *d_wx = d_wz + g.nz, *d_wy = d_wx + g.nx;
+  float *d_wz = at<float>(base, o_t), *d_wx = d_wz + nzt, *d_wy = d_wx + g.nx;
   float *rec = at<float>(base, o_rec);
   unsigned int *mx = at<unsigned int>(base, o_mx);
 
@@ -2785,7 +2670,7 @@ static int run_noalloc(const pw_afd_args *a, const float *vel, const float *src,
       PW_CUDA(cudaStreamSynchronize(st));
     }
   }
-  taper_table_kernel<<<ceil_div(g.nz, 256), 256, 0, st>>>(d_w, p.nb, g.nz, p.nz2, d_wz);
+  taper_table_kernel<<<ceil_div(nzt, 256), 256, 0, st>>>(d_w, p.nb, nzt, p.nz2, d_wz);
   if (two_d) {
     taper_table_kernel<<<1, 32, 0, st>>>(d_w, 0, 1, 1, d_wx);  // dummy axis: factor 1
     taper_table_kernel<<<ceil_div(g.ny, 256), 256, 0, st>>>(d_w, p.nb, g.ny, p.nx2, d_wy);
@@ -2803,11 +2688,10 @@ static int run_noalloc(const pw_afd_args *a, const float *vel, const float *src,
   s.g = g;
   s.ych = p.ych;
   s.ngroups = 1;
+  s.zig = zigzag_pays(3 * nfield * 4);
   s.S = p.S;
-  s.ZS = p.ZS;
-  s.KX = p.KX;
   s.nzc = p.nzc;
-  s.WPC = p.WPC;
+  s.nq = p.nq;
   s.WZ = p.WZ;
   s.WX = p.WX;
   {
@@ -2840,6 +2724,7 @@ static int run_noalloc(const pw_afd_args *a, const float *vel, const float *src,
     s.sx[i] = ksx[i];
     s.sy[i] = ksy[i];
   }
+  source_box(s);
   s.rick = wavelet;
   s.rz = p.nb + a->gz;
   if (two_d) {
@@ -2854,7 +2739,6 @@ static int run_noalloc(const pw_afd_args *a, const float *vel, const float *src,
   s.nz1 = p.knz1; s.nx1 = p.knx1; s.ny1 = p.kny1;
   s.img = nullptr;
   void *fn = p.fn;
-  const int threads = p.threads;
   for (int it = 0; it < nt; it++) {
     s.it = it;
     s.cur[0] = A;
@@ -2863,7 +2747,7 @@ static int run_noalloc(const pw_afd_args *a, const float *vel, const float *src,
     s.wfd = (snap && wfd) ? wfd + (size_t)(it / a->jsnap) * nvel : nullptr;
     void *args[] = {(void *)&s};
     void *f = s.wfd ? p.fn_snap : fn;
-    PW_CUDA(cudaLaunchKernel(f, p.grid, dim3(threads), args, p.smem, st));
+    PW_CUDA(launch_step(f, p, args, st));
     std::swap(A, B);
   }
   if (dat) {

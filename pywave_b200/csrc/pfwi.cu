@@ -60,8 +60,7 @@ struct PfArgs {
   float one;                  // 1.0f at run time: keeps packed products unfused (pk2 helpers)
   DivC divx, divz;            // fast exact division by dx2 / dz2
   float xlo, xhi;             // numerators that both divide as they are
-  int nz4;                    // float4 per padded column
-  unsigned div_m, div_s;      // n / nz4 = umulhi(n, div_m) >> div_s for n < 2^31
+  FastDiv nz4;                // float4 per padded column
   int src_z0, src_z1;         // rows of the shots' source cells
   const float *cur;           // the shots' current fields, fstep floats apart
   float *nxt;                 // the shots' previous fields, overwritten with the next
@@ -69,6 +68,7 @@ struct PfArgs {
   const float *V;             // v*v*dt^2 (field layout)
   const float *bz, *bx;       // sponge factor per z / x cell (1 off the faces)
   int it, nt;
+  int zig;                    // 1: odd steps run their blocks backwards
   const ShotGeo *geo;         // [nshots] (device)
   int rz, drv, nr;
   const float *wav;           // forward: wavelet [nt]
@@ -200,10 +200,10 @@ __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast
 template <int MODE, bool PAS>
 __global__ void __launch_bounds__(32 * PF_XW, MODE == ADJ_REF || PAS ? 5 : 6)
     pf_step_kernel(const __grid_constant__ PfArgs a) {
-  const int s = blockIdx.y;
-  const unsigned item = blockIdx.x * 32 + (threadIdx.x & 31);
-  const int chunk = (int)(__umulhi(item, a.div_m) >> a.div_s);  // item / nz4
-  const int z4 = (int)item - chunk * a.nz4;
+  const int s = zigzag(a.it & a.zig, blockIdx.y, gridDim.y);
+  const unsigned item = zigzag(a.it & a.zig, blockIdx.x, gridDim.x) * 32 + (threadIdx.x & 31);
+  const int chunk = fast_div(item, a.nz4);
+  const int z4 = (int)item - chunk * a.nz4.d;
   const int x = chunk * PF_XW + (threadIdx.x >> 5);
   const int iz0 = 4 * z4;
   pdl_wait();
@@ -935,13 +935,14 @@ static int setup(const pw_fwi_args *a, Setup &S, bool passive = false) {
 
 template <int MODE, bool PAS = false>
 static int launch_one(const Setup &S, const PfArgs &p, int nshots, cudaStream_t st) {
-  const long long lanes = (long long)p.nz4 * ceil_div(S.pnx, PF_XW);
+  const long long lanes = (long long)p.nz4.d * ceil_div(S.pnx, PF_XW);
   const dim3 grid((unsigned)ceil_div(lanes, 32), (unsigned)nshots);
   PW_CUDA(launch_pdl(pf_step_kernel<MODE, PAS>, grid, dim3(32 * PF_XW), 0, st, p));
   return PW_OK;
 }
 
-static int launch(const Setup &S, const PfArgs &p, int mode, int nshots, cudaStream_t st) {
+static int launch(const Setup &S, PfArgs &p, int mode, int nshots, cudaStream_t st) {
+  p.zig = zigzag_pays((size_t)(2 * nshots + 1) * S.fstride * 4);
   if (mode == FWD)
     return p.dsrc ? launch_one<FWD, true>(S, p, nshots, st) : launch_one<FWD>(S, p, nshots, st);
   if (mode == ADJ_REF) return launch_one<ADJ_REF>(S, p, nshots, st);
@@ -968,18 +969,7 @@ static void base_args(const Setup &S, PfArgs &p) {
   p.drv = S.drv;
   p.nr = S.nr;
   p.fstep = S.fstride;
-  p.nz4 = ceil_div(S.pnz, 4);
-  // m = ceil(2^(32 + k) / nz4) with 2^k >= nz4 divides every n < 2^31 exactly
-  // where m fits 32 bits (nz4 > 1); with nz4 = 1 the halved form is n itself
-  int k = 0;
-  while ((1 << k) < p.nz4) k++;
-  if (k == 0) {
-    p.div_m = 0xffffffffu;
-    p.div_s = 0;
-  } else {
-    p.div_m = (unsigned)(((1ull << (31 + k)) + p.nz4 - 1) / p.nz4);
-    p.div_s = k - 1;
-  }
+  p.nz4 = make_fast_div(ceil_div(S.pnz, 4));
   p.src_z0 = 1 << 30;
   p.src_z1 = -1;
   for (const ShotGeo &g : S.geo) {

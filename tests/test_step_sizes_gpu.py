@@ -48,3 +48,92 @@ def test_pfwi_step_sizes_bit_exact(oracle, cuda_lib, nz, nx, nb, scale, h):
     ge, J = fwi.gradient(vel, wav, dobs, par, mode="exact", weight=w)
     gx, Jx = oracle.pfwi_gradient_exact(vel, wav, dobs, weight=w.astype(np.float64), **kw)
     assert rel_l2(ge, gx) < 1e-4 and abs(J - Jx) < 1e-4 * Jx
+
+
+# 2-D step per launch (the resident kernel switched off): depths around 1, 2, 31 .. 33 float4,
+# widths around the 4 columns of a CTA
+@pytest.mark.parametrize("nz,nx,nbt", [(3, 2, 0), (5, 9, 1), (60, 37, 4), (100, 13, 14),
+                                       (101, 18, 14), (103, 31, 15)])
+def test_afd2d_step_sizes_bit_exact(oracle, cuda_lib, monkeypatch, nz, nx, nbt):
+    import pywave_b200 as pw
+    monkeypatch.setenv("PW_AFD_RESIDENT", "0")
+    nt = 60
+    rng = np.random.default_rng(nz * 100 + nx)
+    vel = (1500 + 1500 * rng.random((nz, nx))).astype(np.float32)
+    kw = dict(nt=nt, dt=0.001, ax=[0, 10, nx], az=[0, 10, nz], nbt=nbt, ct=0.02, jsnap=7)
+    s1 = dict(sx=[nx // 2], sz=[nz // 2], f=[30.0], t=[0.01], A=[2.0])
+    if nbt >= 1:
+        d, w = pw.afd2d(vel, ns=1, **s1, **kw)
+        do, wo = oracle.afd(vel, nt, 0.001, (10.0, 10.0), nbt=nbt, ct=0.02, src=s1, jsnap=7)
+        assert np.array_equal(d, do) and np.array_equal(w, wo)
+    tr = rng.standard_normal((nt, nx)).astype(np.float32)
+    _, w = pw.afd2d(vel, dat=tr, tri=True, **kw)
+    _, wo = oracle.afd(vel, nt, 0.001, (10.0, 10.0), nbt=nbt, ct=0.02, tri=True, dat=tr, jsnap=7)
+    assert np.abs(wo).max() > 0 and np.array_equal(w, wo)
+
+
+@pytest.mark.parametrize("nz,nx,ny,nbt", [(3, 2, 3, 0), (7, 5, 6, 2), (58, 11, 9, 3),
+                                          (100, 6, 5, 14), (103, 9, 4, 13)])
+def test_afd3d_step_sizes_bit_exact(oracle, cuda_lib, nz, nx, ny, nbt):
+    import pywave_b200 as pw
+    nt = 40
+    rng = np.random.default_rng(nz * 100 + nx)
+    vel = (1500 + 1500 * rng.random((nz, nx, ny))).astype(np.float32)
+    kw = dict(nt=nt, dt=0.001, ax=[0, 10, nx], ay=[0, 10, ny], az=[0, 10, nz], nbt=nbt, ct=0.02,
+              jsnap=9)
+    s2 = dict(sx=[nx // 2, nx - 1], sy=[ny // 2, 0], sz=[nz // 2, 1], f=[30.0, 25.0],
+              t=[0.01, 0.004], A=[2.0, 1.0])
+    if nbt >= 1:
+        d, w = pw.afd3d(vel, ns=2, **s2, **kw)
+        do, wo = oracle.afd(vel, nt, 0.001, (10.0,) * 3, nbt=nbt, ct=0.02, src=s2, jsnap=9)
+        assert np.array_equal(d, do) and np.array_equal(w, wo)
+    tr = rng.standard_normal((nt, nx, ny)).astype(np.float32)
+    _, w = pw.afd3d(vel, dat=tr, tri=True, **kw)
+    _, wo = oracle.afd(vel, nt, 0.001, (10.0,) * 3, nbt=nbt, ct=0.02, tri=True, dat=tr, jsnap=9)
+    assert np.abs(wo).max() > 0 and np.array_equal(w, wo)
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_tri_image_groups_equal_single_runs(cuda_lib, monkeypatch, dim):
+    """The image formed inside the step (3 groups in lockstep) against the
+    product of three time reversals' snapshots, in group order."""
+    import pywave_b200 as pw
+    monkeypatch.setenv("PW_AFD_RESIDENT", "0")
+    rng = np.random.default_rng(dim)
+    nt, js, G = 90, 5, 3
+    shape = (33, 30) if dim == 2 else (33, 18, 7)
+    vel = (1500 + 1500 * rng.random(shape)).astype(np.float32)
+    tr = rng.standard_normal((nt,) + shape[1:]).astype(np.float32)
+    grp = rng.integers(-1, G, shape[:0:-1]).astype(np.int32).reshape(-1, shape[1])  # [ny, nx]
+    kw = dict(dt=0.001, nbt=6, ct=0.02, jsnap=js)
+    img = pw.tri_image(vel, tr, d=(10.0,) * dim, ngroups=G, groups=grp, normalize=False, **kw)
+    prod = None
+    ax = dict(ax=[0, 10, shape[1]], az=[0, 10, shape[0]])
+    if dim == 3:
+        ax["ay"] = [0, 10, shape[2]]
+    for g in range(G):
+        m = (grp == g).T if dim == 3 else (grp[0] == g)
+        _, w = (pw.afd2d if dim == 2 else pw.afd3d)(vel, nt=nt, dat=(tr * m).astype(np.float32),
+                                                    tri=True, **ax, **kw)
+        prod = w * w if prod is None else prod * w * w
+    ref = np.zeros(shape, np.float32)
+    for k in range(prod.shape[-1] - 1, -1, -1):  # time reversal: the last snapshot comes first
+        ref += prod[..., k]
+    assert np.abs(ref).max() > 0 and np.array_equal(img, ref)
+
+
+def test_batch_of_more_shots_than_the_constant_table(cuda_lib):
+    import pywave_b200 as pw
+    from pywave_b200.afd import afd2d_batch
+    rng = np.random.default_rng(5)
+    shots = []
+    for k in range(101):
+        nz, nx, nt = 12 + k % 7, 10 + k % 5, 20 + k % 9
+        shots.append(dict(vel=(1500 + 900 * rng.random((nz, nx))).astype(np.float32), nt=nt,
+                          dt=0.001, ax=[0, 10.0, nx], az=[0, 10.0, nz], ns=1, sx=[nx // 2],
+                          sz=[nz // 2], f=[30.0], t=[0.005], A=[1.0], nbt=5, ct=0.02, gz=0))
+    got = afd2d_batch(shots)
+    for k, sh in enumerate(shots):
+        kw = {n: sh[n] for n in ("nt", "dt", "ax", "az", "ns", "sx", "sz", "f", "t", "A", "nbt", "ct")}
+        ref = pw.afd2d(sh["vel"], jsnap=0, **kw).reshape(sh["nt"], sh["ax"][2], order="F")
+        assert np.abs(ref).max() > 0 and np.array_equal(got[k], ref), k
