@@ -103,17 +103,6 @@ __device__ __forceinline__ long long pfoff(int lz, int iz, int ix) {
   return (long long)(iz + HZ) + (long long)lz * (ix + HX);
 }
 
-__device__ __forceinline__ void cp16(float4 *dst, const float *src, bool valid) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(dst);
-  const int n = valid ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(src), "r"(n)
-               : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-__device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-
 // largest / smallest |x| of three (a NaN wins the maximum)
 __device__ __forceinline__ float max3abs(float a, float b, float c) {
   float r;
@@ -180,6 +169,10 @@ __device__ __forceinline__ void div4_sum(const f2 (&tx)[2], const f2 (&tz)[2], c
   t[1] = hi2(r);
 }
 
+__device__ __forceinline__ void pdl_sync() {
+  pdl_wait();
+  pdl_launch();
+}
 __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 
 // One pfwi step: a thread updates one float4 of z cells (z4) of one x plane of
@@ -206,8 +199,7 @@ __global__ void __launch_bounds__(32 * PF_XW, MODE == ADJ_REF || PAS ? 5 : 6)
   const int z4 = (int)item - chunk * a.nz4.d;
   const int x = chunk * PF_XW + (threadIdx.x >> 5);
   const int iz0 = 4 * z4;
-  pdl_wait();
-  pdl_launch();
+  pdl_sync();
   if (x >= a.pnx) return;
   const long long lz = a.lz;
   const long long o0 = pfoff(a.lz, iz0, x);  // own float4
@@ -590,9 +582,6 @@ __global__ void transpose_kernel(const float *in, float *out, long long rows, lo
   }
 }
 
-// Exact gradient: dJ/dv_pad = 2 * sum(phi*term) / v_pad, folded back through
-// pad2d's edge replication onto the interior (one thread per interior cell,
-// summing the padded cells that copy it, in a fixed order).
 // (float)(-2./temp) with temp = v*v*v in float (wave_fwigradient.c:224-226),
 // once per call instead of per cell and step
 __global__ void m2v3_kernel(const float *vel, size_t n, float *out) {
@@ -603,19 +592,49 @@ __global__ void m2v3_kernel(const float *vel, size_t n, float *out) {
   }
 }
 
-__global__ void fold_grad_kernel(const float *gacc, const float *vel, int nz, int nx, int nb,
-                                 int pnz, int pnx, int lz, float *grad) {
-  const long long n = (long long)nz * nx;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int jz = int(i % nz), jx = int(i / nz);
+// Sum of a value per thread over a block of 256, in a fixed tree (thread 0's result).
+__device__ __forceinline__ double block_sum(double v) {
+  __shared__ double part[8];
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double s = 0.0;
+  if (threadIdx.x == 0)
+    for (int k = 0; k < 8; k++) s += part[k];
+  return s;
+}
+
+// Exact gradient: dJ/dv_pad = 2 * sum(phi*term) / v_pad, folded back through
+// pad2d's edge replication onto the interior (the padded cells that copy an
+// interior cell, summed in FP64 in a fixed order).
+// Blocks 0 .. 3 sum the corner cells ((nb + 1)^2 padded cells each, 160 us
+// for one thread at nb 60), the others every other cell, one per thread.
+__global__ void __launch_bounds__(256) fold_grad_kernel(const float *gacc, const float *vel, int nz,
+                                                        int nx, int nb, int pnz, int pnx, int lz,
+                                                        float *grad) {
+  if (blockIdx.x < 4) {
+    const int jz = (blockIdx.x & 1) ? nz - 1 : 0, jx = (blockIdx.x & 2) ? nx - 1 : 0;
     const int z_lo = jz == 0 ? 0 : jz + nb, z_hi = jz == nz - 1 ? pnz - 1 : jz + nb;
     const int x_lo = jx == 0 ? 0 : jx + nb, x_hi = jx == nx - 1 ? pnx - 1 : jx + nb;
-    const double v = vel[i];
+    const int cz = z_hi - z_lo + 1, n = cz * (x_hi - x_lo + 1);
+    double s = 0.0;
+    for (int k = threadIdx.x; k < n; k += 256)
+      s += (double)gacc[pfoff(lz, z_lo + k % cz, x_lo + k / cz)];
+    s = block_sum(s);
+    const long long i = (long long)jx * nz + jz;
+    if (threadIdx.x == 0) grad[i] = (float)(2.0 * s / (double)vel[i]);
+    return;
+  }
+  const long long n = (long long)nz * nx;
+  for (long long i = (blockIdx.x - 4) * 256LL + threadIdx.x; i < n; i += (gridDim.x - 4) * 256LL) {
+    const int jz = int(i % nz), jx = int(i / nz);
+    if ((jz == 0 || jz == nz - 1) && (jx == 0 || jx == nx - 1)) continue;
+    const int z_lo = jz == 0 ? 0 : jz + nb, z_hi = jz == nz - 1 ? pnz - 1 : jz + nb;
+    const int x_lo = jx == 0 ? 0 : jx + nb, x_hi = jx == nx - 1 ? pnx - 1 : jx + nb;
     double s = 0.0;
     for (int ix = x_lo; ix <= x_hi; ix++)
       for (int iz = z_lo; iz <= z_hi; iz++) s += (double)gacc[pfoff(lz, iz, ix)];
-    grad[i] = (float)(2.0 * s / v);
+    grad[i] = (float)(2.0 * s / (double)vel[i]);
   }
 }
 
@@ -1519,7 +1538,7 @@ static int gradient_impl(const pw_fwi_args *a, int mode, const float *vel, const
   }
   timer.stop();
   if (exact) {
-    fold_grad_kernel<<<592, 256, 0, st>>>(gacc, d_vel, nz, nx, a->nb, S.pnz, S.pnx, S.lz, gdev);
+    fold_grad_kernel<<<4 + 592, 256, 0, st>>>(gacc, d_vel, nz, nx, a->nb, S.pnz, S.pnx, S.lz, gdev);
     PW_CUDA(cudaGetLastError());
   }
   PW_TRY(to_host(grad, gdev, nvel * 4, host, st));
@@ -2112,8 +2131,7 @@ using pf::FWD;
 using pf::ADJ_EXACT;
 constexpr int MAXS3 = 16;    // shots per launch
 constexpr int MAXSRC = 64;   // source-map cells per shot
-constexpr int XT = 16;       // columns per CTA
-constexpr int NR = 3;        // ring planes (plane y, y + 1, y + 2 in flight)
+constexpr int XW3 = 4;       // columns (warps) per CTA, of one plane
 
 struct Shot {
   int nsrc;
@@ -2125,12 +2143,15 @@ struct Shot {
 struct Args {
   int pnz, pnx, pny, lz;
   long long sx, sy, fstride;
-  int nz4, ZT, nzc, ych;
+  FastDiv nz4;          // float4 per padded column
+  int zig;              // 1: odd steps run their blocks backwards
+  int src_z0, src_z1;   // rows of the shots' source cells
   float c0, c1, c2, c3, c4, rdx2, rdz2, rdy2;
   float one;  // 1.0f at run time: keeps packed products unfused (pk2 helpers)
   int nshots;
-  const float *cur[MAXS3];
-  float *nxt[MAXS3];
+  const float *cur;          // the shots' current fields, fstep floats apart
+  float *nxt;                // the shots' previous fields, overwritten with the next
+  long long fstep;
   const float *V;
   const float *bz, *bx, *by;
   int it, nt;
@@ -2152,208 +2173,148 @@ __host__ __device__ inline long long off3(const Args &a, int iz, int ix, int iy)
   return (long long)(iz + 4) + a.sx * (ix + 4) + a.sy * (iy + 4);
 }
 
-// One step over the CTA's ZT float4 x XT column tile, marching y: the tile of
-// plane y (with a 1-float4 z halo and 4 halo columns each side) is staged in
-// a 3-plane cp.async ring with one CTA barrier per plane; the y neighbours
-// come from a 9-deep register queue of the thread's own float4.
+// One 3-D step: a thread updates one float4 of z cells of one column and plane
+// of one shot, straight from global memory (8 x and 8 y neighbour float4s, the
+// two z neighbours, the previous field and V; for the adjoint the forward term
+// and the gradient), as the 2-D step does.  Shots are the fastest block index,
+// so the shots of a cell share V through L2.
+// Bound: L2 to L1 traffic and load latency (21 float4 loads per float4; DRAM
+// would allow 57 us forward and 80 us adjoint).  Measured, one launch, 2 shots
+// of 160 x 240 x 240, average of forward and adjoint: 95.6 us (157 with the
+// former 3-plane shared-memory ring and a barrier per plane); 1 shot of 200 x
+// 340 x 340 124 us (190), of 100 x 120 x 120 9.9 us (33).  72 registers (28
+// warps per SM): 64 (spills) 102, 80 100, 96 104, 114 112; CTAs of 8 columns
+// 107, of 4 columns x 2 planes 106, x 4 planes 143.
 template <int MODE>
-__global__ void __launch_bounds__(512) pf3_step_kernel(const __grid_constant__ Args a) {
-  extern __shared__ float4 sm3[];
-  constexpr int NST = MODE == FWD ? 2 : 4;  // own streams: prev, V (, term, gradient)
-  const int ZT = a.ZT, TZ = ZT + 2, TX = XT + 8;
-  const int nthr = ZT * XT;
-  const int tid = threadIdx.x, zt = tid % ZT, xt = tid / ZT;
-  const int s = blockIdx.z;
-  const int zc = blockIdx.x % a.nzc, xc = blockIdx.x / a.nzc;
-  const int z4 = zc * ZT + zt, x = xc * XT + xt;
-  const int y0 = blockIdx.y * a.ych, y1 = min(a.pny, y0 + a.ych);
-  const bool live = z4 < a.nz4 && x < a.pnx;
+__global__ void __launch_bounds__(32 * XW3, 7) pf3_step_kernel(const __grid_constant__ Args a) {
+  const int tile = blockIdx.x / a.nshots, s = blockIdx.x - tile * a.nshots;
+  const unsigned item = tile * 32 + (threadIdx.x & 31);
+  const int chunk = fast_div(item, a.nz4);
+  const int z4 = (int)item - chunk * a.nz4.d;
+  const int x = chunk * XW3 + (threadIdx.x >> 5), y = zigzag(a.it & a.zig, blockIdx.y, gridDim.y);
   const int iz0 = 4 * z4;
-  const int tile_n = TZ * TX, slot_n = tile_n + NST * nthr;
-  const float *cur = a.cur[s];
-  float *nxt = a.nxt[s];
-  const float *tin = MODE == ADJ_EXACT ? a.tin + s * a.tin_stride : nullptr;
-  float *gs = MODE == ADJ_EXACT ? a.grad + s * a.gstride : nullptr;
-  const long long sy = a.sy;
-  // own float4 in plane 0 (a safe in-range cell for idle threads)
-  const long long o0 = live ? off3(a, iz0, x, 0) : off3(a, 0, 0, 0);
-  // tile copies: element e = tid + k nthr of the TZ x TX tile, tz fastest
-  constexpr int MAXCP = 4;  // TZ * TX <= 4 * nthr for ZT >= 4
-  long long cpo[MAXCP];
-  bool cok[MAXCP];
+  pf::pdl_sync();
+  if (x >= a.pnx) return;
+  const long long sx = a.sx, sy = a.sy;
+  const long long o = (iz0 + 4) + (long long)((unsigned long long)(unsigned)sx * (unsigned)(x + 4)) +
+                      (long long)((unsigned long long)(unsigned)sy * (unsigned)(y + 4));
+  const float *pc = a.cur + s * a.fstep + o;
+  float *pn = a.nxt + s * a.fstep + o;
+  const float4 c = pf::ld4(pc), L = pf::ld4(pc - 4), R = pf::ld4(pc + 4);
+  float4 xp[4], xm[4], yp[4], ym[4];
 #pragma unroll
-  for (int k = 0; k < MAXCP; k++) {
-    const int e = tid + k * nthr;
-    const int tz = e % TZ, tx = e / TZ;
-    const int zz = zc * ZT - 1 + tz, col = xc * XT - 4 + tx;
-    // the float4 at 4 zz + 4 must lie in the column, the column in the halo
-    cok[k] = e < tile_n && zz >= -1 && 4 * zz + 8 <= a.lz && col >= -4 && col < a.pnx + 4;
-    cpo[k] = cok[k] ? (long long)(4 * zz + 4) + a.sx * (col + 4) + sy * 4 : 0;
+  for (int d = 0; d < 4; d++) {
+    xp[d] = pf::ld4(pc + (d + 1) * sx);
+    xm[d] = pf::ld4(pc - (d + 1) * sx);
   }
-  auto issue = [&](int p, int rs) {  // plane p into ring slot rs
-    if (p < y1) {
-      float4 *dst = sm3 + rs * slot_n;
-      const long long py = sy * p;
 #pragma unroll
-      for (int k = 0; k < MAXCP; k++) {
-        const int e = tid + k * nthr;
-        if (e < tile_n) pf::cp16(dst + e, cur + (cok[k] ? cpo[k] + py : 0), cok[k]);
-      }
-      float4 *own = dst + tile_n + tid;
-      pf::cp16(own, nxt + o0 + py, live);
-      pf::cp16(own + nthr, a.V + o0 + py, live);
-      if (MODE == ADJ_EXACT) {
-        pf::cp16(own + 2 * nthr, tin + o0 + py, live);
-        pf::cp16(own + 3 * nthr, gs + o0 + py, live);
-      }
+  for (int d = 0; d < 4; d++) {
+    yp[d] = pf::ld4(pc + (d + 1) * sy);
+    ym[d] = pf::ld4(pc - (d + 1) * sy);
+  }
+  const float4 pv = pf::ld4(pn), V4 = pf::ld4(a.V + o);
+  float4 tf = make_float4(0.f, 0.f, 0.f, 0.f), g0 = tf;
+  float *pg = nullptr;
+  if (MODE == ADJ_EXACT) {
+    tf = __ldcs(reinterpret_cast<const float4 *>(a.tin + s * a.tin_stride + o));
+    pg = a.grad + s * a.gstride + o;
+    g0 = pf::ld4(pg);
+  }
+  const float bxf = a.bx[x], byf = a.by[y];
+  const float4 bz4 = pf::ld4(a.bz + iz0);
+  const bool lxy = x >= 4 && x < a.pnx - 4 && y >= 4 && y < a.pny - 4;
+  // the stencil's rows [4, pnz - 4): see the 2-D step
+  const bool lz_any = z4 >= 1 && iz0 < a.pnz - 4;
+  const bool full = lxy && lz_any && iz0 + 3 < a.pnz - 4;
+  const f2 k1 = pk2(a.one, a.one);
+  float4 term4;
+  {
+    // the 8th-order sums along x, z and y in the reference's order, and
+    // (tx / dx^2 + tz / dz^2) + ty / dy^2, for cells (0, 1) and (2, 3)
+    // of the float4 per f32x2 op; the z neighbours at odd distances are
+    // the float4s shifted by one cell
+    const f2 kc[5] = {pk2(a.c0, a.c0), pk2(a.c1, a.c1), pk2(a.c2, a.c2), pk2(a.c3, a.c3),
+                      pk2(a.c4, a.c4)};
+    const f2 rx2 = pk2(a.rdx2, a.rdx2), rz2 = pk2(a.rdz2, a.rdz2), ry2 = pk2(a.rdy2, a.rdy2);
+    const f2 cl = lo2(c), ch = hi2(c);
+    const f2 s_wx = pk2(L.w, c.x), s_yz = pk2(c.y, c.z), s_wR = pk2(c.w, R.x);
+    const f2 s_Lyz = pk2(L.y, L.z), s_Ryz = pk2(R.y, R.z);
+    const f2 zp[2][4] = {{s_yz, ch, s_wR, lo2(R)}, {s_wR, lo2(R), s_Ryz, hi2(R)}};
+    const f2 zm[2][4] = {{s_wx, hi2(L), s_Lyz, lo2(L)}, {s_yz, cl, s_wx, hi2(L)}};
+    f2 t2[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      auto P = [h](const float4 &v) { return h ? hi2(v) : lo2(v); };
+      f2 tx = mul2(mul2(kc[0], P(c)), k1), tz = tx, ty = tx;
+#pragma unroll
+      for (int d = 1; d <= 4; d++)
+        tx = add2(tx, mul2(mul2(kc[d], add2(P(xp[d - 1]), P(xm[d - 1]))), k1));
+#pragma unroll
+      for (int d = 1; d <= 4; d++)
+        tz = add2(tz, mul2(mul2(kc[d], add2(zp[h][d - 1], zm[h][d - 1])), k1));
+#pragma unroll
+      for (int d = 1; d <= 4; d++)
+        ty = add2(ty, mul2(mul2(kc[d], add2(P(yp[d - 1]), P(ym[d - 1]))), k1));
+      const f2 sxz = add2(mul2(mul2(tx, rx2), k1), mul2(mul2(tz, rz2), k1));
+      t2[h] = add2(sxz, mul2(mul2(ty, ry2), k1));
     }
-    pf::cp_commit();
-  };
-
-  float bzf[4];
-  bool lz_ok[4], zin[4];
-#pragma unroll
-  for (int e = 0; e < 4; e++) {
-    const int iz = iz0 + e;
-    bzf[e] = (live && iz < a.pnz) ? a.bz[iz] : 1.f;
-    lz_ok[e] = iz >= 4 && iz < a.pnz - 4;
-    zin[e] = iz < a.pnz;
+    term4 = join2(t2[0], t2[1]);
   }
-  const float bxf = live ? a.bx[x] : 1.f;
-  const bool lx_ok = x >= 4 && x < a.pnx - 4;
-  const bool rec_row = live && a.rz >= iz0 && a.rz < iz0 + 4;
-  const int rx_i = rec_row ? a.rxmap[x] : -1;
-  const Shot &sh = a.shots[s];
-  const bool src_zx = MODE == FWD && live && iz0 <= sh.sz1 && iz0 + 3 >= sh.sz0 && x >= sh.sx0 &&
-                      x <= sh.sx1;
-  const int ci = (xt + 4) * TZ + zt + 1;  // own float4 in the tile
-
-  // y queue: q[k] = own float4 of plane y - 4 + k
-  float4 q[9];
-  const float *pc = cur + o0;
+  if (!full) {
 #pragma unroll
-  for (int k = 0; k < 8; k++) q[k] = __ldg(reinterpret_cast<const float4 *>(pc + sy * (y0 - 4 + k)));
-  float4 qn = __ldg(reinterpret_cast<const float4 *>(pc + sy * (y0 + 4)));
-  issue(y0, 0);
-  issue(y0 + 1, 1);
-  int rs = 0;  // ring slot of plane y
-  for (int y = y0; y < y1; y++) {
-    pf::cp_wait<1>();
-    __syncthreads();  // plane y staged; every thread is done with plane y - 1
-    issue(y + 2, rs == 0 ? 2 : rs - 1);  // into the slot plane y - 1 left
-    q[8] = qn;
-    if (y + 1 < y1) qn = __ldg(reinterpret_cast<const float4 *>(pc + sy * (y + 5)));
-    const float4 *tile = sm3 + rs * slot_n;
-    const float4 *own = tile + tile_n + tid;
-    if (live) {
-      const float4 c = q[4];
-      const float4 L = tile[ci - 1], R = tile[ci + 1];
-      const float4 xm1 = tile[ci - TZ], xp1 = tile[ci + TZ];
-      const float4 xm2 = tile[ci - 2 * TZ], xp2 = tile[ci + 2 * TZ];
-      const float4 xm3 = tile[ci - 3 * TZ], xp3 = tile[ci + 3 * TZ];
-      const float4 xm4 = tile[ci - 4 * TZ], xp4 = tile[ci + 4 * TZ];
-      const float4 pv = own[0], V4 = own[nthr];
-      const float byf = a.by[y];
-      const bool ly_ok = y >= 4 && y < a.pny - 4;
-      const long long o = o0 + sy * y;
-      int trace = -1;
-      if (rec_row && rx_i >= 0) {
-        const int ry_j = a.rymap[y];
-        if (ry_j >= 0) trace = ry_j * a.nrx + rx_i;
-      }
-      if (MODE == FWD && trace >= 0 && a.rec)
-        a.rec[((size_t)s * a.nt + a.it) * a.nr + trace] = pf::el(c, a.rz - iz0);
-      const bool src_here = src_zx && y >= sh.sy0 && y <= sh.sy1;
-      float4 term4, res4, lap4;
-      const f2 k1 = pk2(a.one, a.one);
-      {
-        // the 8th-order sums along x, z and y in the reference's order, and
-        // (tx / dx^2 + tz / dz^2) + ty / dy^2, for cells (0, 1) and (2, 3)
-        // of the float4 per f32x2 op; the z neighbours at odd distances are
-        // the float4s shifted by one cell
-        const f2 kc[5] = {pk2(a.c0, a.c0), pk2(a.c1, a.c1), pk2(a.c2, a.c2), pk2(a.c3, a.c3),
-                          pk2(a.c4, a.c4)};
-        const f2 rx2 = pk2(a.rdx2, a.rdx2), rz2 = pk2(a.rdz2, a.rdz2), ry2 = pk2(a.rdy2, a.rdy2);
-        const f2 cl = lo2(c), ch = hi2(c);
-        const f2 s_wx = pk2(L.w, c.x), s_yz = pk2(c.y, c.z), s_wR = pk2(c.w, R.x);
-        const f2 s_Lyz = pk2(L.y, L.z), s_Ryz = pk2(R.y, R.z);
-        const f2 zp[2][4] = {{s_yz, ch, s_wR, lo2(R)}, {s_wR, lo2(R), s_Ryz, hi2(R)}};
-        const f2 zm[2][4] = {{s_wx, hi2(L), s_Lyz, lo2(L)}, {s_yz, cl, s_wx, hi2(L)}};
-        const float4 *xp[4] = {&xp1, &xp2, &xp3, &xp4}, *xm[4] = {&xm1, &xm2, &xm3, &xm4};
-        f2 t2[2];
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const f2 cv2 = h ? ch : cl;
-          f2 tx = mul2(mul2(kc[0], cv2), k1), tz = tx, ty = tx;
-#pragma unroll
-          for (int d = 1; d <= 4; d++) {
-            const f2 xs = h ? add2(hi2(*xp[d - 1]), hi2(*xm[d - 1]))
-                            : add2(lo2(*xp[d - 1]), lo2(*xm[d - 1]));
-            tx = add2(tx, mul2(mul2(kc[d], xs), k1));
-          }
-#pragma unroll
-          for (int d = 1; d <= 4; d++)
-            tz = add2(tz, mul2(mul2(kc[d], add2(zp[h][d - 1], zm[h][d - 1])), k1));
-#pragma unroll
-          for (int d = 1; d <= 4; d++) {
-            const f2 ys = h ? add2(hi2(q[4 + d]), hi2(q[4 - d])) : add2(lo2(q[4 + d]), lo2(q[4 - d]));
-            ty = add2(ty, mul2(mul2(kc[d], ys), k1));
-          }
-          const f2 sxz = add2(mul2(mul2(tx, rx2), k1), mul2(mul2(tz, rz2), k1));
-          t2[h] = add2(sxz, mul2(mul2(ty, ry2), k1));
-        }
-        lap4 = join2(t2[0], t2[1]);
-      }
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        float t = (lz_ok[e] && lx_ok && ly_ok) ? pf::el(lap4, e) : 0.f;
-        const int iz = iz0 + e;
-        if (MODE == FWD) {
-          if (src_here) {
-            const int key = iz | (x << 11) | (y << 22);
-            for (int k = 0; k < sh.nsrc; k++)
-              if (sh.scell[k] == key) t = fadd(t, fmul(sh.sw[k], a.wav[a.it]));
-          }
-        } else if (trace >= 0 && iz == a.rz) {
-          t = fadd(t, a.res[((size_t)s * a.nt + a.it) * a.nr + trace]);
-        }
-        pf::set_el(term4, e, t);
-      }
-      {
-        // taper of the stored u_{k-1} (z, then x, then y faces), the update
-        // with 2 c as c + c (the same bits, no product to fuse), the taper
-        const f2 bx2 = pk2(bxf, bxf), by2 = pk2(byf, byf);
-        f2 r2[2];
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const f2 bz2 = pk2(bzf[2 * h], bzf[2 * h + 1]);
-          const f2 cv2 = h ? hi2(c) : lo2(c);
-          const f2 p = mul2(mul2(by2, mul2(bx2, mul2(bz2, h ? hi2(pv) : lo2(pv)))), k1);
-          const f2 vt = mul2(mul2(h ? hi2(V4) : lo2(V4), h ? hi2(term4) : lo2(term4)), k1);
-          const f2 v = add2(sub2(add2(cv2, cv2), p), vt);
-          r2[h] = mul2(by2, mul2(bx2, mul2(bz2, v)));
-        }
-        res4 = join2(r2[0], r2[1]);
+    for (int e = 0; e < 4; e++)
+      if (!(lxy && lz_any && iz0 + e < a.pnz - 4)) pf::set_el(term4, e, 0.f);
+  }
+  if (a.rz >= iz0 && a.rz < iz0 + 4) {
+    // receivers: traces read the field before the step, residuals enter the adjoint
+    const int rx_i = a.rxmap[x], ry_j = a.rymap[y];
+    if (rx_i >= 0 && ry_j >= 0) {
+      const size_t k = ((size_t)s * a.nt + a.it) * a.nr + (ry_j * a.nrx + rx_i);
+      if (MODE == FWD) {
+        if (a.rec) a.rec[k] = pf::el(c, a.rz - iz0);
+      } else {
+        const float r = a.res[k];
 #pragma unroll
         for (int e = 0; e < 4; e++)
-          if (!zin[e]) pf::set_el(res4, e, 0.f);
-      }
-      *reinterpret_cast<float4 *>(nxt + o) = res4;
-      if (MODE == FWD && a.tout)
-        *reinterpret_cast<float4 *>(a.tout + s * a.tout_stride + o) = term4;
-      if (MODE == ADJ_EXACT) {
-        const float4 tf = own[2 * nthr];
-        const float4 g0 = own[3 * nthr];
-        const float4 g = join2(add2(lo2(g0), mul2(mul2(lo2(c), lo2(tf)), k1)),
-                               add2(hi2(g0), mul2(mul2(hi2(c), hi2(tf)), k1)));
-        *reinterpret_cast<float4 *>(gs + o) = g;
+          if (iz0 + e == a.rz) pf::set_el(term4, e, fadd(pf::el(term4, e), r));
       }
     }
-#pragma unroll
-    for (int k = 0; k < 8; k++) q[k] = q[k + 1];
-    rs = rs == 2 ? 0 : rs + 1;
   }
-  pf::cp_wait_all();
+  if (MODE == FWD && iz0 <= a.src_z1 && iz0 + 3 >= a.src_z0) {
+    const Shot &sh = a.shots[s];
+    if (x >= sh.sx0 && x <= sh.sx1 && y >= sh.sy0 && y <= sh.sy1) {
+      const float wv = a.wav[a.it];
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        const int key = (iz0 + e) | (x << 11) | (y << 22);
+        for (int k = 0; k < sh.nsrc; k++)
+          if (sh.scell[k] == key)
+            pf::set_el(term4, e, fadd(pf::el(term4, e), fmul(sh.sw[k], wv)));
+      }
+    }
+  }
+  {
+    // taper of the stored u_{k-1} (z, then x, then y faces), the update
+    // with 2 c as c + c (the same bits, no product to fuse), the taper;
+    // cells beyond pnz stay zero: every operand is zero there
+    const f2 bx2 = pk2(bxf, bxf), by2 = pk2(byf, byf);
+    f2 r2[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const f2 bz2 = h ? hi2(bz4) : lo2(bz4);
+      const f2 cv2 = h ? hi2(c) : lo2(c);
+      const f2 p = mul2(mul2(by2, mul2(bx2, mul2(bz2, h ? hi2(pv) : lo2(pv)))), k1);
+      const f2 vt = mul2(mul2(h ? hi2(V4) : lo2(V4), h ? hi2(term4) : lo2(term4)), k1);
+      const f2 v = add2(sub2(add2(cv2, cv2), p), vt);
+      r2[h] = mul2(by2, mul2(bx2, mul2(bz2, v)));
+    }
+    *reinterpret_cast<float4 *>(pn) = join2(r2[0], r2[1]);
+  }
+  if (MODE == FWD && a.tout)
+    __stcs(reinterpret_cast<float4 *>(a.tout + s * a.tout_stride + o), term4);
+  if (MODE == ADJ_EXACT)
+    *reinterpret_cast<float4 *>(pg) = join2(add2(lo2(g0), mul2(mul2(lo2(c), lo2(tf)), k1)),
+                                            add2(hi2(g0), mul2(mul2(hi2(c), hi2(tf)), k1)));
 }
 
 // V = (v v) dt^2 on the padded grid (edge replication on every face)
@@ -2371,20 +2332,61 @@ __global__ void pad_V3_kernel(const float *vel, int nz, int nx, int ny, int nb, 
 }
 
 // dJ/dv = 2 / v * sum of the accumulators of the padded cells that pad3d
-// copies from the interior cell (edge replication adjoint)
-__global__ void fold_grad3_kernel(const float *gacc, const float *vel, int nz, int nx, int ny,
-                                  int nb, Args g, float *grad) {
-  const long long n = (long long)nz * nx * ny;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int jz = int(i % nz), jx = int((i / nz) % nx), jy = int(i / ((long long)nz * nx));
-    const int z_lo = jz == 0 ? 0 : jz + nb, z_hi = jz == nz - 1 ? g.pnz - 1 : jz + nb;
-    const int x_lo = jx == 0 ? 0 : jx + nb, x_hi = jx == nx - 1 ? g.pnx - 1 : jx + nb;
-    const int y_lo = jy == 0 ? 0 : jy + nb, y_hi = jy == ny - 1 ? g.pny - 1 : jy + nb;
+// copies from the interior cell (edge replication adjoint).  The first
+// `edges` blocks take one edge or corner cell each ((nb + 1)^2 or (nb + 1)^3
+// padded cells; one thread per cell took 1.1 ms at nb 20), the others every
+// other cell, one per thread.
+__device__ __forceinline__ void fold_range(int j, int n, int pn, int nb, int &lo, int &hi) {
+  lo = j == 0 ? 0 : j + nb;
+  hi = j == n - 1 ? pn - 1 : j + nb;
+}
+__global__ void __launch_bounds__(256) fold_grad3_kernel(const float *gacc, const float *vel, int nz,
+                                                         int nx, int ny, int nb, Args g,
+                                                         float *grad, int edges) {
+  int z0, z1, x0, x1, y0, y1;
+  if ((int)blockIdx.x < edges) {
+    // block 4 k + corner: along y (k < ny), then x, then z
+    const int corner = blockIdx.x & 3;
+    int k = blockIdx.x >> 2, jz, jx, jy;
+    if (k < ny) {
+      jy = k;
+      jz = (corner & 1) ? nz - 1 : 0;
+      jx = (corner & 2) ? nx - 1 : 0;
+    } else if (k < ny + nx) {
+      jx = k - ny;
+      jz = (corner & 1) ? nz - 1 : 0;
+      jy = (corner & 2) ? ny - 1 : 0;
+    } else {
+      jz = k - ny - nx;
+      jx = (corner & 1) ? nx - 1 : 0;
+      jy = (corner & 2) ? ny - 1 : 0;
+    }
+    fold_range(jz, nz, g.pnz, nb, z0, z1);
+    fold_range(jx, nx, g.pnx, nb, x0, x1);
+    fold_range(jy, ny, g.pny, nb, y0, y1);
+    const int cz = z1 - z0 + 1, cx = x1 - x0 + 1;
+    const long long n = (long long)cz * cx * (y1 - y0 + 1);
     double s = 0.0;
-    for (int iy = y_lo; iy <= y_hi; iy++)
-      for (int ix = x_lo; ix <= x_hi; ix++)
-        for (int iz = z_lo; iz <= z_hi; iz++) s += (double)gacc[off3(g, iz, ix, iy)];
+    for (long long q = threadIdx.x; q < n; q += 256)
+      s += (double)gacc[off3(g, z0 + (int)(q % cz), x0 + (int)(q / cz % cx), y0 + (int)(q / cz / cx))];
+    s = pf::block_sum(s);
+    const size_t i = ((size_t)jy * nx + jx) * nz + jz;
+    if (threadIdx.x == 0) grad[i] = (float)(2.0 * s / (double)vel[i]);
+    return;
+  }
+  const long long n = (long long)nz * nx * ny;
+  for (long long i = (blockIdx.x - edges) * 256LL + threadIdx.x; i < n;
+       i += (gridDim.x - edges) * 256LL) {
+    const int jz = int(i % nz), jx = int((i / nz) % nx), jy = int(i / ((long long)nz * nx));
+    const int faces = (jz == 0 || jz == nz - 1) + (jx == 0 || jx == nx - 1) + (jy == 0 || jy == ny - 1);
+    if (faces >= 2) continue;
+    fold_range(jz, nz, g.pnz, nb, z0, z1);
+    fold_range(jx, nx, g.pnx, nb, x0, x1);
+    fold_range(jy, ny, g.pny, nb, y0, y1);
+    double s = 0.0;
+    for (int iy = y0; iy <= y1; iy++)
+      for (int ix = x0; ix <= x1; ix++)
+        for (int iz = z0; iz <= z1; iz++) s += (double)gacc[off3(g, iz, ix, iy)];
     grad[i] = (float)(2.0 * s / (double)vel[i]);
   }
 }
@@ -2454,10 +2456,8 @@ static int setup3(const pw_fwi3d_args *a, Setup3 &S) {
   g.sx = g.lz;
   g.sy = (long long)g.lz * (g.pnx + 8);
   g.fstride = g.sy * (g.pny + 8) + 64;
-  g.nz4 = ceil_div(g.pnz, 4);
-  const int nzc = ceil_div(g.nz4, 32);
-  g.ZT = std::max(4, ceil_div(g.nz4, nzc));
-  g.nzc = ceil_div(g.nz4, g.ZT);
+  g.nz4 = make_fast_div(ceil_div(g.pnz, 4));
+  g.fstep = g.fstride;
   const float c0 = -205. / 72, c1 = 8. / 5, c2 = -1. / 5, c3 = 8. / 315, c4 = -1. / 560;
   g.c0 = c0; g.c1 = c1; g.c2 = c2; g.c3 = c3; g.c4 = c4;
   g.rdz2 = 1.f / (a->dz * a->dz);
@@ -2476,6 +2476,7 @@ static int setup3(const pw_fwi3d_args *a, Setup3 &S) {
     for (int i = n - nb; i < n; i++) f[i] = bc[n - i - 1];
   };
   axis(g.pnz, S.bz);
+  S.bz.resize(round_up(g.pnz, 4), 1.f);  // read four at a time
   axis(g.pnx, S.bx);
   axis(g.pny, S.by);
   // receivers: the nrx x nry grid (rx[i], ry[j]) at depth rz, trace j nrx + i
@@ -2503,46 +2504,22 @@ static int setup3(const pw_fwi3d_args *a, Setup3 &S) {
              "shot %d: source (z=%d, x=%d, y=%d) outside the model", is, z, x, y);
     PW_TRY(source_map3(z + nb, x + nb, y + nb, S, S.shots[is]));
   }
-  return PW_OK;
-}
-
-static size_t smem3(const Args &g, int mode) {
-  const int nthr = g.ZT * XT;
-  const int slot = (g.ZT + 2) * (XT + 8) + (mode == FWD ? 2 : 4) * nthr;
-  return (size_t)NR * slot * sizeof(float4);
-}
-
-template <int MODE>
-static int launch3_t(const Args &p, cudaStream_t st) {
-  const size_t smem = smem3(p, MODE);
-  static bool attr = false;
-  if (!attr) {
-    int dev = 0, maxsm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    cudaFuncSetAttribute(pf3_step_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm);
-    cudaGetLastError();
-    attr = true;
+  g.src_z0 = 1 << 30;
+  g.src_z1 = -1;
+  for (const Shot &sh : S.shots) {
+    g.src_z0 = std::min(g.src_z0, sh.sz0);
+    g.src_z1 = std::max(g.src_z1, sh.sz1);
   }
-  const dim3 grid((unsigned)(p.nzc * ceil_div(p.pnx, XT)), (unsigned)ceil_div(p.pny, p.ych),
-                  (unsigned)p.nshots);
-  pf3_step_kernel<MODE><<<grid, p.ZT * XT, smem, st>>>(p);
-  PW_CUDA(cudaGetLastError());
   return PW_OK;
 }
-static int launch3(const Args &p, int mode, cudaStream_t st) {
-  return mode == FWD ? launch3_t<FWD>(p, st) : launch3_t<ADJ_EXACT>(p, st);
-}
 
-// planes per CTA: enough CTAs for every SM a few times over
-static int plan_ych(const Args &g, int nshots) {
-  int dev = 0, nsm = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const long long cols = (long long)g.nzc * ceil_div(g.pnx, XT) * nshots;
-  int ych = g.pny;
-  while (ych > 16 && cols * ceil_div(g.pny, ych) < 8LL * nsm) ych = (ych + 1) / 2;
-  return ych;
+static int launch3(Args &p, int mode, cudaStream_t st) {
+  p.zig = zigzag_pays((size_t)(2 * p.nshots + 1) * p.fstride * 4);
+  const long long lanes = (long long)p.nz4.d * ceil_div(p.pnx, XW3);
+  const dim3 grid((unsigned)(ceil_div(lanes, 32) * p.nshots), (unsigned)p.pny);
+  PW_CUDA(launch_pdl(mode == FWD ? pf3_step_kernel<FWD> : pf3_step_kernel<ADJ_EXACT>, grid,
+                     dim3(32 * XW3), 0, st, p));
+  return PW_OK;
 }
 
 }  // namespace pf3
@@ -2659,26 +2636,19 @@ extern "C" int pw_pfwi3d_forward(const pw_fwi3d_args *a, const float *vel, const
   long long launches = 0;
   for (int s0 = 0; s0 < ns; s0 += nsb) {
     const int nb_ = std::min(nsb, ns - s0);
-    float *A[MAXS3], *B[MAXS3];
-    for (int s = 0; s < nb_; s++) {
-      A[s] = at<float>(base, b.o_A) + s * fs;
-      B[s] = at<float>(base, b.o_B) + s * fs;
-    }
-    PW_CUDA(cudaMemsetAsync(base + b.o_A, 0, (size_t)nsb * fs * 4, st));
-    PW_CUDA(cudaMemsetAsync(base + b.o_B, 0, (size_t)nsb * fs * 4, st));
+    float *A = at<float>(base, b.o_A), *B = at<float>(base, b.o_B);
+    PW_CUDA(cudaMemsetAsync(A, 0, (size_t)nsb * fs * 4, st));
+    PW_CUDA(cudaMemsetAsync(B, 0, (size_t)nsb * fs * 4, st));
     p.nshots = nb_;
     p.shots = at<Shot>(base, b.o_shots) + s0;
     p.rec = rec + (size_t)s0 * nt * nr;
-    p.ych = plan_ych(S.g, nb_);
     for (int it = 0; it < nt; it++) {
       p.it = it;
-      for (int s = 0; s < nb_; s++) {
-        p.cur[s] = A[s];
-        p.nxt[s] = B[s];
-      }
+      p.cur = A;
+      p.nxt = B;
       PW_TRY(launch3(p, FWD, st));
       launches++;
-      for (int s = 0; s < nb_; s++) std::swap(A[s], B[s]);
+      std::swap(A, B);
     }
   }
   timer.stop();
@@ -2774,16 +2744,21 @@ extern "C" int pw_pfwi3d_gradient(const pw_fwi3d_args *a, const float *vel, cons
   long long launches = 0;
   for (int s0 = 0; s0 < ns; s0 += nsb) {
     const int nb_ = std::min(nsb, ns - s0);
-    float *A[MAXS3], *B[MAXS3];
-    for (int s = 0; s < nb_; s++) {
-      A[s] = at<float>(base, b.o_A) + s * fs;
-      B[s] = at<float>(base, b.o_B) + s * fs;
-    }
-    PW_CUDA(cudaMemsetAsync(base + b.o_A, 0, (size_t)nsb * fs * 4, st));
-    PW_CUDA(cudaMemsetAsync(base + b.o_B, 0, (size_t)nsb * fs * 4, st));
+    float *A = at<float>(base, b.o_A), *B = at<float>(base, b.o_B);
+    PW_CUDA(cudaMemsetAsync(A, 0, (size_t)nsb * fs * 4, st));
+    PW_CUDA(cudaMemsetAsync(B, 0, (size_t)nsb * fs * 4, st));
     p.nshots = nb_;
     p.shots = at<Shot>(base, b.o_shots) + s0;
-    p.ych = plan_ych(S.g, nb_);
+    auto step = [&](int mode, int it, float *&cur, float *&nxt, size_t stride) -> int {
+      p.it = it;
+      p.cur = cur;
+      p.nxt = nxt;
+      p.fstep = (long long)stride;
+      PW_TRY(launch3(p, mode, st));
+      launches++;
+      std::swap(cur, nxt);
+      return PW_OK;
+    };
     float *dd = at<float>(base, o_d), *res = at<float>(base, o_res);
     float *ck = at<float>(base, o_ck), *tb = at<float>(base, o_tb);
     // ---- forward: traces, checkpoints, the last segment's terms
@@ -2795,19 +2770,12 @@ extern "C" int pw_pfwi3d_gradient(const pw_fwi3d_args *a, const float *vel, cons
         const int m = it / k;
         for (int s = 0; s < nb_; s++) {
           float *c = ck + ((size_t)s * nck + m) * 2 * fs;
-          PW_CUDA(cudaMemcpyAsync(c, A[s], fs * 4, cudaMemcpyDeviceToDevice, st));
-          PW_CUDA(cudaMemcpyAsync(c + fs, B[s], fs * 4, cudaMemcpyDeviceToDevice, st));
+          PW_CUDA(cudaMemcpyAsync(c, A + s * fs, fs * 4, cudaMemcpyDeviceToDevice, st));
+          PW_CUDA(cudaMemcpyAsync(c + fs, B + s * fs, fs * 4, cudaMemcpyDeviceToDevice, st));
         }
       }
       p.tout = it >= n_last ? tb + (size_t)(it - n_last) * fs : nullptr;
-      p.it = it;
-      for (int s = 0; s < nb_; s++) {
-        p.cur[s] = A[s];
-        p.nxt[s] = B[s];
-      }
-      PW_TRY(launch3(p, FWD, st));
-      launches++;
-      for (int s = 0; s < nb_; s++) std::swap(A[s], B[s]);
+      PW_TRY(step(FWD, it, A, B, fs));
     }
     p.rec = nullptr;
     p.tout = nullptr;
@@ -2818,43 +2786,22 @@ extern "C" int pw_pfwi3d_gradient(const pw_fwi3d_args *a, const float *vel, cons
     PW_CUDA(cudaGetLastError());
     p.res = res;
     // ---- backward by segments (the adjoint pair reuses the forward pair)
-    PW_CUDA(cudaMemsetAsync(base + b.o_A, 0, (size_t)nsb * fs * 4, st));
-    PW_CUDA(cudaMemsetAsync(base + b.o_B, 0, (size_t)nsb * fs * 4, st));
-    float *adjA[MAXS3], *adjB[MAXS3];
-    for (int s = 0; s < nb_; s++) {
-      adjA[s] = at<float>(base, b.o_A) + s * fs;
-      adjB[s] = at<float>(base, b.o_B) + s * fs;
-    }
+    A = at<float>(base, b.o_A);
+    B = at<float>(base, b.o_B);
+    PW_CUDA(cudaMemsetAsync(A, 0, (size_t)nsb * fs * 4, st));
+    PW_CUDA(cudaMemsetAsync(B, 0, (size_t)nsb * fs * 4, st));
     p.tin_stride = (long long)k * fs;
     for (int m = nck - 1; m >= 0; m--) {
       const int n0 = m * k, n1 = std::min(nt, n0 + k);
-      float *FA[MAXS3], *FB[MAXS3];
-      for (int s = 0; s < nb_; s++) {
-        FA[s] = ck + ((size_t)s * nck + m) * 2 * fs;
-        FB[s] = FA[s] + fs;
-      }
+      float *FA = ck + (size_t)m * 2 * fs, *FB = FA + fs;
       for (int n = n0; n < n1 && m < nck - 1; n++) {  // the last segment is kept
-        p.it = n;
-        for (int s = 0; s < nb_; s++) {
-          p.cur[s] = FA[s];
-          p.nxt[s] = FB[s];
-        }
         p.tout = tb + (size_t)(n - n0) * fs;
-        PW_TRY(launch3(p, FWD, st));
-        launches++;
-        for (int s = 0; s < nb_; s++) std::swap(FA[s], FB[s]);
+        PW_TRY(step(FWD, n, FA, FB, (size_t)nck * 2 * fs));
       }
       p.tout = nullptr;
       for (int n = n1 - 1; n >= n0; n--) {
-        p.it = n;
-        for (int s = 0; s < nb_; s++) {
-          p.cur[s] = adjA[s];
-          p.nxt[s] = adjB[s];
-        }
         p.tin = tb + (size_t)(n - n0) * fs;
-        PW_TRY(launch3(p, ADJ_EXACT, st));
-        launches++;
-        for (int s = 0; s < nb_; s++) std::swap(adjA[s], adjB[s]);
+        PW_TRY(step(ADJ_EXACT, n, A, B, fs));
       }
     }
     p.tin = nullptr;
@@ -2867,7 +2814,9 @@ extern "C" int pw_pfwi3d_gradient(const pw_fwi3d_args *a, const float *vel, cons
   }
   timer.stop();
   float *gdev = at<float>(base, o_grad);
-  fold_grad3_kernel<<<592, 256, 0, st>>>(gacc, d_vel, a->nz, a->nx, a->ny, a->nb, S.g, gdev);
+  const int edges = 4 * (a->nz + a->nx + a->ny);
+  fold_grad3_kernel<<<edges + 592, 256, 0, st>>>(gacc, d_vel, a->nz, a->nx, a->ny, a->nb, S.g, gdev,
+                                                 edges);
   PW_CUDA(cudaGetLastError());
   PW_TRY(to_host(grad, gdev, nvel * 4, host, st));
   if (misfit) PW_CUDA(cudaMemcpyAsync(misfit, dmis, 8, cudaMemcpyDeviceToHost, st));

@@ -137,3 +137,26 @@ def test_batch_of_more_shots_than_the_constant_table(cuda_lib):
         kw = {n: sh[n] for n in ("nt", "dt", "ax", "az", "ns", "sx", "sz", "f", "t", "A", "nbt", "ct")}
         ref = pw.afd2d(sh["vel"], jsnap=0, **kw).reshape(sh["nt"], sh["ax"][2], order="F")
         assert np.abs(ref).max() > 0 and np.array_equal(got[k], ref), k
+
+
+# padded depths of 15, 20, 128 (32 float4), 130 and 131 cells; widths off the 4 columns of a CTA
+@pytest.mark.parametrize("nz,nx,ny,nb,ns", [(5, 6, 5, 5, 1), (8, 9, 7, 6, 3), (112, 7, 6, 8, 1),
+                                            (114, 6, 7, 8, 2), (115, 9, 5, 8, 1)])
+def test_pfwi3d_step_sizes(oracle, cuda_lib, nz, nx, ny, nb, ns):
+    from pywave_b200 import fwi3d
+    nt = 70
+    rng = np.random.default_rng(nz * 10 + nx)
+    vt = (1.8 + 0.8 * rng.random((nz, nx, ny))).astype(np.float32)
+    wav = (1e6 * _pulse(nt, 0.001, 40.0)).astype(np.float32)
+    geom = dict(nb=nb, coef=0.02, dz=0.01, dx=0.012, dy=0.011, nt=nt, dt=0.001,
+                src=[(nz // 2, (i * 2) % nx, i % ny) for i in range(ns)], rz=nz // 2,
+                rx=list(range(0, nx, 2)), ry=list(range(ny)))
+    d = fwi3d.forward3d(vt, wav, geom)
+    d32 = oracle.pf3_forward(vt, wav, geom, "f32")
+    assert np.abs(d32).max() > 0 and np.array_equal(d.view(np.uint32), d32.view(np.uint32))
+    dobs = (0.5 * d32).astype(np.float32)
+    # 2 x 70 steps of float32 (6e-8 each) against FP64, the residual half the data; edges and
+    # corners fold (nb + 1)^2 and (nb + 1)^3 padded cells
+    g, J = fwi3d.gradient3d(vt, wav, dobs, geom)
+    go, Jo = oracle.pf3_gradient_exact(vt, wav, dobs, geom)
+    assert rel_l2(g, go) < 1e-4 and abs(J - Jo) < 1e-4 * Jo
