@@ -209,9 +209,19 @@ constexpr int QW2 = 4;           // 2-D: columns (warps) per CTA
 
 __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 
+__device__ __forceinline__ void square_into(float4 &prod, const float4 &u) {
+  prod.x = fmul(fmul(prod.x, u.x), u.x);
+  prod.y = fmul(fmul(prod.y, u.y), u.y);
+  prod.z = fmul(fmul(prod.z, u.z), u.z);
+  prod.w = fmul(fmul(prod.w, u.w), u.w);
+}
+
+// Groups [g0, g1) of one float4; the square product of their new values in
+// group order multiplies `prod` (imaging steps).
 template <bool XT, bool TRI, bool SNAP>
 __device__ __forceinline__ void quad_update(const StepArgs &a, int slot, int ix, int y, int it,
-                                            bool swap) {
+                                            bool swap, int g0, int g1, float4 &prod,
+                                            float4 *last = nullptr) {
   const Geo &g = a.g;
   const int iz0 = 4 * slot - HZ;
   const long long sx = g.sx, sy = g.sy;
@@ -242,10 +252,8 @@ __device__ __forceinline__ void quad_update(const StepArgs &a, int slot, int ix,
     }
   }
   const bool in_xy = SNAP && ix >= a.nbx && ix < a.nbx + a.nx1 && y >= a.nby && y < a.nby + a.ny1;
-  float4 prod = make_float4(1.f, 1.f, 1.f, 1.f);
-  const int G = TRI ? a.ngroups : 1;
 #pragma unroll 1
-  for (int gi = 0; gi < G; gi++) {
+  for (int gi = TRI ? g0 : 0; gi < (TRI ? g1 : 1); gi++) {
     const float *A = (swap ? a.nxt[gi] : a.cur[gi]) + o;
     float *B = (swap ? const_cast<float *>(a.cur[gi]) : a.nxt[gi]) + o;
     const float4 c = ld4(A), pv = ld4(B);
@@ -301,20 +309,25 @@ __device__ __forceinline__ void quad_update(const StepArgs &a, int slot, int ix,
         if (iz0 + e >= a.nbz && iz0 + e < a.nbz + a.nz1) w[e] = el(res, e);
     }
     if (SNAP && TRI) {
-      prod.x = fmul(fmul(prod.x, res.x), res.x);
-      prod.y = fmul(fmul(prod.y, res.y), res.y);
-      prod.z = fmul(fmul(prod.z, res.z), res.z);
-      prod.w = fmul(fmul(prod.w, res.w), res.w);
+      square_into(prod, res);
+      if (last) *last = res;
     }
   }
-  if (SNAP && TRI && a.img && in_xy && iz0 + 3 >= a.nbz && iz0 < a.nbz + a.nz1) {
-    // the demos' image (test_third_tri.py:71-77): img += prod_g u_g^2
-    float4 im = ld4(a.img + o);
+}
+
+// The demos' image (test_third_tri.py:71-77) of one float4: img += prod_g u_g^2.
+__device__ __forceinline__ void quad_image(const StepArgs &a, int slot, int ix, int y,
+                                           const float4 &prod) {
+  const int iz0 = 4 * slot - HZ;
+  if (!a.img || ix < a.nbx || ix >= a.nbx + a.nx1 || y < a.nby || y >= a.nby + a.ny1 ||
+      iz0 + 3 < a.nbz || iz0 >= a.nbz + a.nz1)
+    return;
+  float *p = a.img + 4LL * slot + a.g.sx * (ix + a.g.hx) + a.g.sy * (y + a.g.hy);
+  float4 im = ld4(p);
 #pragma unroll
-    for (int e = 0; e < 4; e++)
-      if (iz0 + e >= a.nbz && iz0 + e < a.nbz + a.nz1) set_el(im, e, fadd(el(im, e), el(prod, e)));
-    *reinterpret_cast<float4 *>(a.img + o) = im;
-  }
+  for (int e = 0; e < 4; e++)
+    if (iz0 + e >= a.nbz && iz0 + e < a.nbz + a.nz1) set_el(im, e, fadd(el(im, e), el(prod, e)));
+  *reinterpret_cast<float4 *>(p) = im;
 }
 
 // lane -> (column group, slot): lanes are numbered nq * group + slot - 1, so
@@ -370,18 +383,37 @@ __global__ void __launch_bounds__(32 * QXW, 6)
   const int y = zigzag(a.it & a.zig, blockIdx.z * gridDim.y + blockIdx.y, gridDim.y * gridDim.z);
   const bool live = ix < a.g.nx && y < a.g.ny;
   if (a.stats != nullptr) quad_stats<TRI>(a, live, slot, ix, y);
-  if (live) quad_update<true, TRI, SNAP>(a, slot, ix, y, a.it, false);
+  if (!live) return;
+  float4 prod = make_float4(1.f, 1.f, 1.f, 1.f);
+  quad_update<true, TRI, SNAP>(a, slot, ix, y, a.it, false, 0, a.ngroups, prod);
+  if (SNAP && TRI) quad_image(a, slot, ix, y, prod);
 }
 
-// 2-D: QW2 columns of the kernel's y (the model's x) per CTA
+// 2-D: QW2 columns of the kernel's y (the model's x) per CTA, and one warp per
+// column and group (a 2-D step is a chain of load latencies: the groups in
+// turn in one thread took 4.8 us per step of 261^2 and 4 groups, in warps of
+// their own 2D4G).  The image product meets the groups in shared memory.
 template <bool TRI, bool SNAP>
-__global__ void __launch_bounds__(32 * QW2) quad2_kernel(const __grid_constant__ StepArgs a) {
+__global__ void __launch_bounds__(32 * QW2 * (TRI ? MAXG : 1))
+    quad2_kernel(const __grid_constant__ StepArgs a) {
+  __shared__ float4 fac[SNAP && TRI ? 32 * QW2 * MAXG : 1];
   int group;
   const int slot = quad_slot(a, zigzag(a.it & a.zig, blockIdx.x, gridDim.x), group);
-  const int y = group * QW2 + (threadIdx.x >> 5);
+  const int w = threadIdx.x >> 5, gi = TRI ? w / QW2 : 0, y = group * QW2 + (TRI ? w % QW2 : w);
   pdl_wait();
   pdl_launch();
-  if (y < a.g.ny) quad_update<false, TRI, SNAP>(a, slot, 0, y, a.it, false);
+  const bool live = y < a.g.ny;
+  float4 prod = make_float4(1.f, 1.f, 1.f, 1.f), u;
+  if (live) quad_update<false, TRI, SNAP>(a, slot, 0, y, a.it, false, gi, gi + 1, prod, &u);
+  if (SNAP && TRI) {
+    fac[threadIdx.x] = u;
+    __syncthreads();
+    if (live && gi == 0) {
+      prod = make_float4(1.f, 1.f, 1.f, 1.f);
+      for (int k = 0; k < a.ngroups; k++) square_into(prod, fac[threadIdx.x + 32 * QW2 * k]);
+      quad_image(a, slot, 0, y, prod);
+    }
+  }
 }
 
 // Cluster-resident 2-D propagation for grids that fit in the distributed
@@ -395,9 +427,17 @@ __global__ void __launch_bounds__(32 * QW2) quad2_kernel(const __grid_constant__
 // stores), and ends with one cluster barrier; the next step reads the halos
 // locally.  Domain edges keep zero halos, as the global layout does.  The
 // arithmetic per cell is quad_update's, term by term, so results are
-// bit-identical to the step-per-launch path.
+// bit-identical to the step-per-launch path.  Bound: the latency of one step
+// (about 130 instructions of a warp, then a cluster barrier of 0.3 us that
+// also waits for the step's stores).  Measured, us per step: 141^2 forward 1.1
+// (1.85 with samples loaded and traces stored in global memory every step and
+// masks and sources tested per cell), 201^2 1.6 (2.6), 261^2 2.1 (3.0).
 constexpr int RES_NTH = 512;   // threads per CTA
 constexpr int RES_MAXIPT = 8;  // items (float4 of z cells) per thread, at most
+constexpr int RES_MAXWORK = 20480;  // float4s (of all groups) a cluster is given, see plan_resident
+constexpr int RES_CH = 32;     // steps whose samples are staged in shared memory at a time
+// staged floats: wavelets [MAXSRC][RES_CH], traces or injected samples [RES_CH][w]
+__host__ __device__ constexpr int res_stage(int w) { return (MAXSRC + w) * RES_CH; }
 
 struct ResArgs {
   StepArgs s;    // it, wfd and img are set per step inside the kernel
@@ -446,6 +486,10 @@ __global__ void __launch_bounds__(RES_NTH) resident_kernel(const __grid_constant
   float4 *swz4 = vvs + arr4;
   float *swz = reinterpret_cast<float *>(swz4);
   float *swy = swz + r.LZ;
+  // samples of the coming RES_CH steps, read and written in global memory once
+  // per RES_CH steps: a load of the step's sample, or a store that the cluster
+  // barrier's release has to wait for, is off the step's critical path
+  float *s_rick = swy + w, *s_tr = s_rick + MAXSRC * RES_CH;
   for (int i = threadIdx.x; i < r.LZ; i += blockDim.x)
     swz[i] = (i >= HZ && i - HZ < g.nz) ? a.wz[i - HZ] : 1.f;
   for (int i = threadIdx.x; i < w; i += blockDim.x) swy[i] = y0 + i < g.ny ? a.wy[y0 + i] : 1.f;
@@ -461,11 +505,11 @@ __global__ void __launch_bounds__(RES_NTH) resident_kernel(const __grid_constant
     vvs[i] = v;
   }
   // this thread's items (fixed for the whole run): shared-memory offset, and
-  // flag bits 0 live, 1-4 Laplacian rows, 5-8 kept rows, 9 Laplacian
-  // column, 10 receiver row, 11 source column, 12 interior column, 13/14 edge
+  // flag bits 0 live, 1-4 cell in the Laplacian's region, 9 all four, 10 receiver
+  // row, 11 holds a cell of a source's spread, 12 interior column, 13/14 edge
   // column copied to the left / right neighbour
   const int items = w * r.nsl;
-  int po4[IPT], pc[IPT];
+  int po4[IPT], pc[IPT], pgid[IPT];  // pgid: the group that injects in a receiver cell
   unsigned pf[IPT];
   float4 pwz[IPT];
   float pwy[IPT];
@@ -482,16 +526,17 @@ __global__ void __launch_bounds__(RES_NTH) resident_kernel(const __grid_constant
 #pragma unroll
       for (int e = 0; e < 4; e++) {
         const int iz = iz0 + e;
-        if (iz >= g.lz0 && iz < g.lz1) f |= 2u << e;
-        if (iz < g.nz) f |= 32u << e;
+        if (iz >= g.lz0 && iz < g.lz1 && y >= g.ly0 && y < g.ly1) f |= 2u << e;
       }
-      if (y >= g.ly0 && y < g.ly1) f |= 1u << 9;
+      if ((f & 30u) == 30u) f |= 1u << 9;
       const int erz = a.rz - iz0;
       if (erz >= 0 && erz < 4 && a.rx0 == 0 && a.nrx >= 1 && y >= a.ry0 && y < a.ry0 + a.nry)
         f |= 1u << 10;
       bool sp = false;
       if (!TRI)
-        for (int sidx = 0; sidx < a.ns; sidx++) sp |= (y >= a.sy[sidx] - 1 && y <= a.sy[sidx] + 1);
+        for (int sidx = 0; sidx < a.ns; sidx++)
+          sp |= y >= a.sy[sidx] - 1 && y <= a.sy[sidx] + 1 && iz0 <= a.sz[sidx] + 1 &&
+                iz0 + 3 >= a.sz[sidx] - 1;
       if (sp) f |= 1u << 11;
       if (y >= a.nby && y < a.nby + a.ny1 && 0 >= a.nbx && 0 < a.nbx + a.nx1) f |= 1u << 12;
       if (c < 2 && rank > 0) f |= 1u << 13;
@@ -500,6 +545,7 @@ __global__ void __launch_bounds__(RES_NTH) resident_kernel(const __grid_constant
     po4[j] = (c + 2) * LZ4 + slot;
     pc[j] = c;
     pf[j] = f;
+    pgid[j] = TRI && (f & (1u << 10)) ? (a.gid == nullptr ? 0 : a.gid[(y - a.ry0) * a.nrx]) : -1;
   }
   __syncthreads();  // the taper tables
 #pragma unroll
@@ -511,7 +557,38 @@ __global__ void __launch_bounds__(RES_NTH) resident_kernel(const __grid_constant
   }
   cluster_sync_all();  // every CTA's arrays are zeroed before any halo store
   const int nrec = a.nrx * a.nry;
+  const bool rec_on = !TRI && a.rec != nullptr;
+  // owned columns' receivers: index of column 0 of the band (columns outside the range unused)
+  const int rcol = y0 - a.ry0;
+  auto stage = [&](int k0, bool load) {  // write back the chunk before k0, load the one from k0
+    if (rec_on && k0 > 0) {
+      const int kb = (k0 - 1) / RES_CH * RES_CH;
+      for (int i = threadIdx.x; i < (k0 - kb) * w; i += RES_NTH) {
+        const int j = i / w, c = i - j * w;
+        if ((unsigned)(rcol + c) < (unsigned)a.nry && y0 + c < g.ny)
+          a.rec[(size_t)(kb + j) * nrec + rcol + c] = s_tr[j * w + c];
+      }
+      __syncthreads();
+    }
+    if (!load) return;
+    const int n = min(RES_CH, a.nt - k0);
+    if (TRI) {
+      for (int i = threadIdx.x; i < n * w; i += RES_NTH) {
+        const int j = i / w, c = i - j * w;
+        if ((unsigned)(rcol + c) < (unsigned)a.nry)
+          s_tr[j * w + c] = a.tri_dat[(size_t)(a.nt - 1 - k0 - j) * nrec + rcol + c];
+      }
+    } else {
+      for (int i = threadIdx.x; i < a.ns * n; i += RES_NTH) {
+        const int sidx = i / n, j = i - sidx * n;
+        s_rick[sidx * RES_CH + j] = a.rick[(size_t)sidx * a.nt + k0 + j];
+      }
+    }
+    __syncthreads();
+  };
   for (int k = 0; k < a.nt; k++) {
+    const int kc = k % RES_CH;
+    if (kc == 0) stage(k, true);
     const int it = TRI ? a.nt - 1 - k : k;
     const bool snap = r.jsnap > 0 && it % r.jsnap == 0;
     float *wfd = (snap && r.wfd0) ? r.wfd0 + (size_t)(it / r.jsnap) * r.nvel : nullptr;
@@ -527,12 +604,10 @@ __global__ void __launch_bounds__(RES_NTH) resident_kernel(const __grid_constant
       const int iz0 = 4 * slot - HZ;
       const float wz[4] = {pwz[j].x, pwz[j].y, pwz[j].z, pwz[j].w};
       const float wy = pwy[j];
-      const bool lyok = f & (1u << 9);
       const bool rec_here = f & (1u << 10);
-      const bool src_plane = f & (1u << 11);
       const int erz = a.rz - iz0;
-      const int r_idx = rec_here ? (y - a.ry0) * a.nrx : 0;
       const float4 vv4 = vvs[o4];
+      const f2 k1 = pk2(a.one, a.one);
       float4 prod = make_float4(1.f, 1.f, 1.f, 1.f);
       float4 res0 = make_float4(0.f, 0.f, 0.f, 0.f);
       for (int gi = 0; gi < G; gi++) {
@@ -540,56 +615,52 @@ __global__ void __launch_bounds__(RES_NTH) resident_kernel(const __grid_constant
         float4 *__restrict__ nxt = res_sm + (2 * gi + 1 - par) * arr4;
         const float4 q0 = cur[o4 - 2 * LZ4], q1 = cur[o4 - LZ4], q2 = cur[o4];
         const float4 q3 = cur[o4 + LZ4], q4 = cur[o4 + 2 * LZ4];
-        const float4 L = cur[o4 - 1], R = cur[o4 + 1];
-        const float Lz = L.z, Lw = L.w, Rx = R.x, Ry = R.y;
+        const float2 L = reinterpret_cast<const float2 *>(cur + o4 - 1)[1];
+        const float2 R = reinterpret_cast<const float2 *>(cur + o4 + 1)[0];
         const float4 pv = nxt[o4];
-        bool inj = false;
-        float dval = 0.f;
-        if (TRI && rec_here) {
-          inj = a.gid == nullptr ? gi == 0 : a.gid[r_idx] == gi;
-          if (inj) dval = a.tri_dat[(size_t)it * nrec + r_idx];
+        float4 lap = lap_quad<false>(a, k1, q2, q1, q3, q0, q4, q2, q2, q2, q2, L.x, L.y, R.x, R.y);
+        if (!(f & (1u << 9))) {  // some cell outside the Laplacian's region
+#pragma unroll
+          for (int e = 0; e < 4; e++)
+            if (!(f & (2u << e))) set_el(lap, e, 0.f);
         }
-        const f2 k1 = pk2(a.one, a.one);
-        float4 lap = lap_quad<false>(a, k1, q2, q1, q3, q0, q4, q2, q2, q2, q2, Lz, Lw, Rx, Ry);
-#pragma unroll
-        for (int e = 0; e < 4; e++)
-          if (!((f & (2u << e)) && lyok)) set_el(lap, e, 0.f);
         float4 res = update_quad<false>(k1, q2, pv, lap, vv4, wz, 1.f, wy);
+        if (TRI) {
+          if (pgid[j] == gi) {
+            const float dval = s_tr[kc * w + c];
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const float vve = el(vv4, e);
-          float v = el(res, e);
-          if (TRI) {
-            if (inj && e == erz) v = fadd(v, fmul(vve, dval));
-          } else if (src_plane) {
-            const int iz = iz0 + e;
-            for (int sidx = 0; sidx < a.ns; sidx++) {
-              const int dz = iz - a.sz[sidx], dys = y - a.sy[sidx];
-              if (dz >= -1 && dz <= 1 && dys >= -1 && dys <= 1) {
+            for (int e = 0; e < 4; e++)
+              if (e == erz) set_el(res, e, fadd(el(res, e), fmul(el(vv4, e), dval)));
+          }
+        } else if (f & (1u << 11)) {
+          for (int sidx = 0; sidx < a.ns; sidx++) {
+            const int dys = y - a.sy[sidx];
+            if ((unsigned)(dys + 1) > 2u) continue;
+            const float wv = s_rick[sidx * RES_CH + kc];
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+              const int dz = iz0 + e - a.sz[sidx];
+              if (dz >= -1 && dz <= 1) {
                 const float den = (float)(abs(dys) + abs(dz) + 1);
-                v = fadd(v, fdiv(fmul(vve, a.rick[(size_t)sidx * a.nt + it]), den));
+                set_el(res, e, fadd(el(res, e), fdiv(fmul(el(vv4, e), wv), den)));
               }
             }
           }
-          set_el(res, e, v);
         }
+        // cells beyond nz stay zero: every operand is zero there
         res = taper_quad<false>(res, wz, 1.f, wy);
-#pragma unroll
-        for (int e = 0; e < 4; e++)
-          if (!(f & (32u << e))) set_el(res, e, 0.f);
         nxt[o4] = res;
         // the neighbours' halo copies of the two edge columns
         if (f & (1u << 13)) *dsmem_map(nxt + o4 + w * LZ4, rank - 1) = res;
         if (f & (1u << 14)) *dsmem_map(nxt + o4 - w * LZ4, rank + 1) = res;
-        if (gi == 0) res0 = res;
         if (TRI) {
-          prod.x = fmul(fmul(prod.x, res.x), res.x);
-          prod.y = fmul(fmul(prod.y, res.y), res.y);
-          prod.z = fmul(fmul(prod.z, res.z), res.z);
-          prod.w = fmul(fmul(prod.w, res.w), res.w);
+          if (img) square_into(prod, res);
+          if (wfd && gi == 0) res0 = res;
+        } else {
+          res0 = res;
         }
       }
-      if (!TRI && rec_here && a.rec) a.rec[(size_t)it * nrec + r_idx] = el(res0, erz);
+      if (rec_on && rec_here) s_tr[kc * w + c] = el(res0, erz);
       const bool interior = f & (1u << 12);
       if (wfd && interior) {
 #pragma unroll
@@ -612,6 +683,7 @@ __global__ void __launch_bounds__(RES_NTH) resident_kernel(const __grid_constant
     }
     cluster_sync_all();
   }
+  stage(a.nt, false);
 }
 
 // Batched 2-D forward modelling of shots of uneven size and length: one
@@ -630,13 +702,14 @@ template <bool TAB>
 __global__ void __launch_bounds__(32 * QW2) batch_kernel(const StepArgs *args, const int2 *items,
                                                          int it, int zig) {
   const int2 item = items[zigzag(it & zig, blockIdx.x, gridDim.x)];
+  float4 none;
   int group;
   if constexpr (TAB) {
     const StepArgs &sa = reinterpret_cast<const StepArgs *>(batch_tab)[item.x];
     const int slot = quad_slot(sa, item.y, group), y = group * QW2 + (threadIdx.x >> 5);
     pdl_wait();
     pdl_launch();
-    if (y < sa.g.ny) quad_update<false, false, false>(sa, slot, 0, y, it, (it & 1) != 0);
+    if (y < sa.g.ny) quad_update<false, false, false>(sa, slot, 0, y, it, (it & 1) != 0, 0, 1, none);
   } else {
     __shared__ StepArgs sa;
     const int *src = reinterpret_cast<const int *>(args + item.x);
@@ -647,7 +720,7 @@ __global__ void __launch_bounds__(32 * QW2) batch_kernel(const StepArgs *args, c
     const int slot = quad_slot(sa, item.y, group), y = group * QW2 + (threadIdx.x >> 5);
     pdl_wait();
     pdl_launch();
-    if (y < sa.g.ny) quad_update<false, false, false>(sa, slot, 0, y, it, (it & 1) != 0);
+    if (y < sa.g.ny) quad_update<false, false, false>(sa, slot, 0, y, it, (it & 1) != 0, 0, 1, none);
   }
 }
 
@@ -1457,7 +1530,7 @@ static void plan_quad(bool tri, int G, Plan &p) {
   const long long lanes = (long long)p.nq.d * (two_d ? ceil_div(g.ny, QW2) : ceil_div(g.nx, QXW));
   p.grid = dim3((unsigned)ceil_div(lanes, 32), two_d ? 1u : (unsigned)std::min(g.ny, 65535),
                 two_d ? 1u : (unsigned)ceil_div(g.ny, 65535));
-  p.threads = 32 * (two_d ? QW2 : QXW);
+  p.threads = 32 * (two_d ? QW2 * (tri ? G : 1) : QXW);
   p.smem = 0;
   if (getenv("PW_AFD_VERBOSE"))
     fprintf(stderr, "afd quad plan: G=%d nq=%d threads=%d grid=%ux%u\n", G, p.nq.d, p.threads,
@@ -1746,6 +1819,13 @@ static void *resident_fn(bool tri, int ipt) {
 static bool plan_resident(const Geo &g, int G, bool tri, ResPlan &rp) {
   const char *env = getenv("PW_AFD_RESIDENT");
   if (env && env[0] == '0') return false;
+  // one cluster's 16 SMs against a launch per step on all of them: measured,
+  // us per step, resident / launches: forward 5 K float4s 1.1 / 2.4, 10 K 1.6 /
+  // 2.4, 17 K 2.1 / 2.4, 26 K 2.6 / 2.4; time reversal, float4s of all groups:
+  // 10 K 1.7 / 2.4, 20 K 2.4 / 2.6, 31 K 3.5 / 2.5 (PW_AFD_RESIDENT=1 takes the
+  // cluster wherever the grid fits)
+  const long long work = (long long)(tri ? G : 1) * ceil_div(g.nz, 4) * g.ny;
+  if (work > RES_MAXWORK && !(env && env[0] == '1')) return false;
   int dev = 0, maxsm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
@@ -1759,7 +1839,7 @@ static bool plan_resident(const Geo &g, int G, bool tri, ResPlan &rp) {
     const int ipt = (w * rp.nsl + RES_NTH - 1) / RES_NTH;
     if (ipt > RES_MAXIPT) break;  // smaller clusters only need more
     rp.fn = resident_fn(tri, ipt);
-    const size_t smem = ((size_t)narr * (w + 4) * rp.LZ + rp.LZ + w) * sizeof(float);
+    const size_t smem = ((size_t)narr * (w + 4) * rp.LZ + rp.LZ + w + res_stage(w)) * sizeof(float);
     if (smem > (size_t)maxsm) break;  // smaller clusters only need more
     // the kernel's shared-memory limit only grows (it is per kernel, and a
     // cached smaller value must not shadow a larger one set since); the
