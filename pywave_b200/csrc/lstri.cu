@@ -33,7 +33,7 @@
 //     loaded into registers one step ahead.  Several shots run as separate
 //     clusters of the same launch.
 //   step_kernel: the same per-quad arithmetic on fields in global memory,
-//     one launch per step, for grids too large for a cluster.
+//     one launch per step, for all but small grids.
 #include "pw_common.cuh"
 
 #include <algorithm>
@@ -47,9 +47,10 @@ namespace tr {
 
 constexpr int RNTH = 512;   // resident_kernel: threads per CTA
 constexpr int RMAXIPT = 8;  // resident_kernel: quads per thread, at most
-constexpr int SNTH = 256;   // step_kernel: threads per block
+constexpr int SNTH = 128;   // step_kernel: threads per block
 constexpr int DOTB = 296;   // reduction blocks (2 per SM)
 constexpr int DOTT = 256;   // reduction threads per block
+constexpr int CGU = 8;      // model-side elements per thread in flight
 
 struct Args {
   int nzp, nxp, nq;  // padded sizes; z quads per padded column
@@ -66,6 +67,9 @@ struct Args {
   int w;             // resident_kernel: padded columns per CTA
   const float4 *X;   // step_kernel: A of every shot, [shot][nxp][nq]
   float4 *Y;         // step_kernel: B, overwritten with A'
+  const float4 *W;   // step_kernel, adjoint: A vv of every shot
+  float4 *Wn;        // step_kernel, adjoint: A' vv, the next step's W
+  FastDiv nqd;       // step_kernel: nq
   size_t fstride;    // step_kernel: float4 per shot field
   int it;            // step_kernel: time index of this step
 };
@@ -105,84 +109,73 @@ __device__ __forceinline__ unsigned quad_flags(const Args &a, int ix, int k) {
   return f;
 }
 
-// A' of the quad, two cells per f32x2 op (pk2 helpers).  The 8th-order sums
-// of Lap (ADJ = false: plain samples, the sum times the centre's vv) or LapT
-// (ADJ = true: every sample times its own vv) in the reference's order;
-// ux[4] / vx[4] is the quad's own column, ux[4 +- d] the columns +-d, uzl /
-// uzh (vzl / vzh) the quads below / above.  Every product that is added is
-// multiplied by the runtime 1.0 first, and 2 u is formed as u + u.  Cells
-// outside the stencil stay zero.  inj: modelling, the source samples of the
-// interior cells (mod[it]); adjoint, element 0 the data sample of the data
-// row.
+// A' of the quad, two cells per f32x2 op (pk2 helpers).  The 8th-order sums of
+// Lap (ADJ = false: plain samples, the sum times the centre's vv) or LapT (ADJ
+// = true: every sample times its own vv) in the reference's order over the
+// samples sx9[4 +- d] of the columns +-d and the quads szl / szh below / above
+// the quad's own sx9[4]: A itself, or for LapT the products A vv, each rounded
+// on its own.  Every product that is added is multiplied by the runtime 1.0
+// first, and 2 A is formed as A + A.  Cells outside the stencil stay zero.
+// inj: modelling, the source samples of the interior cells (mod[it]); adjoint,
+// element 0 the data sample of the data row.
 template <bool ADJ>
-__device__ __forceinline__ float4 quad_step(const Args &a, unsigned f, const float4 (&ux)[9],
-                                            const float4 &uzl, const float4 &uzh,
-                                            const float4 (&vx)[9], const float4 &vzl,
-                                            const float4 &vzh, const float4 &B, const float4 &wz4,
+__device__ __forceinline__ float4 quad_step(const Args &a, unsigned f, const float4 (&sx9)[9],
+                                            const float4 &szl, const float4 &szh, const float4 &A,
+                                            const float4 &V, const float4 &B, const float4 &wz4,
                                             float wxv, const float4 &inj, int k) {
   const f2 k1 = pk2(a.one, a.one);
   const f2 kc[5] = {pk2(a.c0, a.c0), pk2(a.c1, a.c1), pk2(a.c2, a.c2), pk2(a.c3, a.c3),
                     pk2(a.c4, a.c4)};
   // z partners (+d, -d), d = 1..4, of each pair of cells: the quads shifted
-  const float4 &c = ux[4], &L = uzl, &R = uzh;
+  const float4 &c = sx9[4], &L = szl, &R = szh;
   const f2 u_yz = pk2(c.y, c.z), u_wx = pk2(L.w, c.x), u_wR = pk2(c.w, R.x);
-  const f2 zpu[2][4] = {{u_yz, hi2(c), u_wR, lo2(R)}, {u_wR, lo2(R), pk2(R.y, R.z), hi2(R)}};
-  const f2 zmu[2][4] = {{u_wx, hi2(L), pk2(L.y, L.z), lo2(L)}, {u_yz, lo2(c), u_wx, hi2(L)}};
-  f2 zpv[2][4], zmv[2][4];
-  if (ADJ) {
-    const float4 &cv = vx[4], &Lv = vzl, &Rv = vzh;
-    const f2 v_yz = pk2(cv.y, cv.z), v_wx = pk2(Lv.w, cv.x), v_wR = pk2(cv.w, Rv.x);
-    const f2 p0[4] = {v_yz, hi2(cv), v_wR, lo2(Rv)}, p1[4] = {v_wR, lo2(Rv), pk2(Rv.y, Rv.z), hi2(Rv)};
-    const f2 m0[4] = {v_wx, hi2(Lv), pk2(Lv.y, Lv.z), lo2(Lv)}, m1[4] = {v_yz, lo2(cv), v_wx, hi2(Lv)};
-#pragma unroll
-    for (int d = 0; d < 4; d++) {
-      zpv[0][d] = p0[d];
-      zpv[1][d] = p1[d];
-      zmv[0][d] = m0[d];
-      zmv[1][d] = m1[d];
-    }
-  }
+  const f2 zp[2][4] = {{u_yz, hi2(c), u_wR, lo2(R)}, {u_wR, lo2(R), pk2(R.y, R.z), hi2(R)}};
+  const f2 zm[2][4] = {{u_wx, hi2(L), pk2(L.y, L.z), lo2(L)}, {u_yz, lo2(c), u_wx, hi2(L)}};
   const f2 sx = pk2(a.sx, a.sx), sz = pk2(a.sz, a.sz), wx2 = pk2(wxv, wxv);
   f2 n2[2];
 #pragma unroll
   for (int h = 0; h < 2; h++) {
     auto P = [h](const float4 &v) { return h ? hi2(v) : lo2(v); };
-    // sample i of the x window and the z sample pair at +-d (times vv for LapT)
-    auto tx = [&](int i) { return ADJ ? mul2(mul2(P(ux[i]), P(vx[i])), k1) : P(ux[i]); };
-    auto tzp = [&](int d) { return ADJ ? mul2(mul2(zpu[h][d - 1], zpv[h][d - 1]), k1) : zpu[h][d - 1]; };
-    auto tzm = [&](int d) { return ADJ ? mul2(mul2(zmu[h][d - 1], zmv[h][d - 1]), k1) : zmu[h][d - 1]; };
-    const f2 t0 = ADJ ? mul2(mul2(P(ux[4]), P(vx[4])), k1) : P(ux[4]);
-    f2 xs = mul2(mul2(kc[4], add2(tx(8), tx(0))), k1);
-    xs = add2(xs, mul2(mul2(kc[3], add2(tx(7), tx(1))), k1));
-    xs = add2(xs, mul2(mul2(kc[2], add2(tx(6), tx(2))), k1));
-    xs = add2(xs, mul2(mul2(kc[1], add2(tx(5), tx(3))), k1));
-    xs = add2(xs, mul2(mul2(kc[0], t0), k1));
-    f2 zs = mul2(mul2(kc[4], add2(tzp(4), tzm(4))), k1);
-    zs = add2(zs, mul2(mul2(kc[3], add2(tzp(3), tzm(3))), k1));
-    zs = add2(zs, mul2(mul2(kc[2], add2(tzp(2), tzm(2))), k1));
-    zs = add2(zs, mul2(mul2(kc[1], add2(tzp(1), tzm(1))), k1));
-    zs = add2(zs, mul2(mul2(kc[0], t0), k1));
+    const f2 t0 = mul2(mul2(kc[0], P(c)), k1);
+    f2 xs = mul2(mul2(kc[4], add2(P(sx9[8]), P(sx9[0]))), k1);
+    xs = add2(xs, mul2(mul2(kc[3], add2(P(sx9[7]), P(sx9[1]))), k1));
+    xs = add2(xs, mul2(mul2(kc[2], add2(P(sx9[6]), P(sx9[2]))), k1));
+    xs = add2(xs, mul2(mul2(kc[1], add2(P(sx9[5]), P(sx9[3]))), k1));
+    xs = add2(xs, t0);
+    f2 zs = mul2(mul2(kc[4], add2(zp[h][3], zm[h][3])), k1);
+    zs = add2(zs, mul2(mul2(kc[3], add2(zp[h][2], zm[h][2])), k1));
+    zs = add2(zs, mul2(mul2(kc[2], add2(zp[h][1], zm[h][1])), k1));
+    zs = add2(zs, mul2(mul2(kc[1], add2(zp[h][0], zm[h][0])), k1));
+    zs = add2(zs, t0);
     f2 lap = add2(mul2(mul2(xs, sx), k1), mul2(mul2(zs, sz), k1));
-    if (!ADJ) lap = mul2(mul2(lap, P(vx[4])), k1);
+    if (!ADJ) lap = mul2(mul2(lap, P(V)), k1);
     const f2 u0 = mul2(mul2(mul2(P(B), P(wz4)), wx2), k1);
-    n2[h] = sub2(add2(lap, add2(P(ux[4]), P(ux[4]))), u0);
+    n2[h] = sub2(add2(lap, add2(P(A), P(A))), u0);
   }
   float4 n = join2(n2[0], n2[1]);
+  if (!ADJ) {
+    if (f & (0xFu << 5)) {
 #pragma unroll
-  for (int e = 0; e < 4; e++) {
-    float v = qel(n, e);
-    if (!ADJ) {
-      if (f & (32u << e)) v = fadd(v, fmul(qel(inj, e), qel(vx[4], e)));
-    } else {
-      if ((f & (1u << 9)) && e == a.depth - 4 * k) v = fadd(v, inj.x);
+      for (int e = 0; e < 4; e++)
+        if (f & (32u << e)) qset(n, e, fadd(qel(n, e), fmul(qel(inj, e), qel(V, e))));
     }
-    qset(n, e, v);
+  } else if (f & (1u << 9)) {
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+      if (e == a.depth - 4 * k) qset(n, e, fadd(qel(n, e), inj.x));
   }
   float4 r = join2(mul2(mul2(lo2(n), lo2(wz4)), wx2), mul2(mul2(hi2(n), hi2(wz4)), wx2));
+  if ((f & 0x1Eu) != 0x1Eu) {
 #pragma unroll
-  for (int e = 0; e < 4; e++)
-    if (!(f & (2u << e))) qset(r, e, 0.f);
+    for (int e = 0; e < 4; e++)
+      if (!(f & (2u << e))) qset(r, e, 0.f);
+  }
   return r;
+}
+// u v per cell, rounded on its own also where it is added next
+__device__ __forceinline__ float4 quad_mul(float one, const float4 &u, const float4 &v) {
+  const f2 k1 = pk2(one, one);
+  return join2(mul2(mul2(lo2(u), lo2(v)), k1), mul2(mul2(hi2(u), hi2(v)), k1));
 }
 
 // the next step's injected samples of one quad
@@ -203,20 +196,20 @@ __device__ __forceinline__ float4 load_inj(const Args &a, const float *mod, cons
 }
 
 // what a step writes besides the fields: modelling records the data row of
-// A (before the step), the adjoint images A vv on the interior
+// A (before the step), the adjoint images A vv on the interior (S: A or A vv)
 template <bool ADJ>
 __device__ __forceinline__ void quad_out(const Args &a, float *mod, float *dat, unsigned f,
-                                         const float4 &A, const float4 &V, int ix, int k, int it) {
+                                         const float4 &S, int ix, int k, int it) {
   if (!ADJ) {
     if (f & (1u << 9)) {
       const int e = a.depth - 4 * k;
-      dat[(size_t)(ix - a.nb) * a.nt + it] = fadd(0.f, qel(A, e));
+      dat[(size_t)(ix - a.nb) * a.nt + it] = fadd(0.f, qel(S, e));
     }
   } else if (f & (0xFu << 5)) {
     const long long row = ((long long)it * a.nx + (ix - a.nb)) * a.nz - a.nb + 4 * k;
 #pragma unroll
     for (int e = 0; e < 4; e++)
-      if (f & (32u << e)) __stcs(mod + row + e, fadd(0.f, fmul(qel(A, e), qel(V, e))));
+      if (f & (32u << e)) __stcs(mod + row + e, fadd(0.f, qel(S, e)));
   }
 }
 
@@ -293,24 +286,19 @@ __global__ void __launch_bounds__(RNTH) resident_kernel(const __grid_constant__ 
       if (!f) continue;
       const int c = (int)((f >> 12) & 1023u), k = (int)(f >> 22), ix = x0 + c;
       const int o = (c + 4) * nq + k;
-      float4 ux[9], vx[9];
+      float4 sx9[9];
 #pragma unroll
-      for (int d = 0; d < 9; d++) ux[d] = cur[o + (d - 4) * nq];
-      const float4 uzl = cur[o - 1], uzh = cur[o + 1];
-      float4 vzl = make_float4(0.f, 0.f, 0.f, 0.f), vzh = vzl;
+      for (int d = 0; d < 9; d++) sx9[d] = cur[o + (d - 4) * nq];
+      float4 szl = cur[o - 1], szh = cur[o + 1];
+      const float4 A = sx9[4], V = Vs[o];
       if (ADJ) {
 #pragma unroll
-        for (int d = 0; d < 9; d++) vx[d] = Vs[o + (d - 4) * nq];
-        vzl = Vs[o - 1];
-        vzh = Vs[o + 1];
-      } else {
-#pragma unroll
-        for (int d = 0; d < 9; d++) vx[d] = vzl;
-        vx[4] = Vs[o];
+        for (int d = 0; d < 9; d++) sx9[d] = quad_mul(a.one, sx9[d], d == 4 ? V : Vs[o + (d - 4) * nq]);
+        szl = quad_mul(a.one, szl, Vs[o - 1]);
+        szh = quad_mul(a.one, szh, Vs[o + 1]);
       }
-      quad_out<ADJ>(a, mod, dat, f, ux[4], vx[4], ix, k, it);
-      const float4 r = quad_step<ADJ>(a, f, ux, uzl, uzh, vx, vzl, vzh, nxt[o], wzs[k], wxs[c],
-                                      inj[j], k);
+      quad_out<ADJ>(a, mod, dat, f, ADJ ? sx9[4] : A, ix, k, it);
+      const float4 r = quad_step<ADJ>(a, f, sx9, szl, szh, A, V, nxt[o], wzs[k], wxs[c], inj[j], k);
       inj[j] = load_inj<ADJ>(a, mod, dat, f, ix, k, ADJ ? it - 1 : it + 1);
       nxt[o] = r;
       if (f & (1u << 10)) *cl_map(nxt + o + w * nq, rank - 1) = r;
@@ -320,39 +308,60 @@ __global__ void __launch_bounds__(RNTH) resident_kernel(const __grid_constant__ 
   }
 }
 
+// One step per launch, a quad per thread straight from L1 / L2; small blocks,
+// so that a shot spreads over all SMs.  The adjoint keeps A vv beside A (W,
+// written by the step that forms A'), so both directions read 9 + 2 sample
+// quads where LapT on A and vv read twice that.  Bound by the latency of
+// dependent launches: what no step writes is read before pdl_wait, and
+// modelling asks L2 for the next step's source samples, which stream from
+// HBM.  130 x 334 with 60 sponge cells, per step: 2.1 us in both directions;
+// before, 4.1 (adjoint, by steps) and 3.9 (modelling, resident).
 template <bool ADJ>
-__global__ void __launch_bounds__(SNTH) step_kernel(const Args a) {
+__global__ void __launch_bounds__(SNTH) step_kernel(const __grid_constant__ Args a) {
   const int shot = blockIdx.y;
-  const long long item = (long long)blockIdx.x * SNTH + threadIdx.x;
-  const int nq = a.nq;
-  const int ix = (int)(item / nq), k = (int)(item - (long long)ix * nq);
-  if (ix >= a.nxp) return;
-  const unsigned f = quad_flags(a, ix, k);
-  if (!f) return;
-  const float4 *__restrict__ X = a.X + (size_t)shot * a.fstride;
-  float4 *__restrict__ Y = a.Y + (size_t)shot * a.fstride;
-  const float4 *__restrict__ V = a.vv;
+  const unsigned item = blockIdx.x * SNTH + threadIdx.x;
+  const int nq = a.nq, ix = fast_div(item, a.nqd), k = (int)item - ix * nq;
+  const unsigned f = ix < a.nxp ? quad_flags(a, ix, k) : 0;
   float *mod = a.mod + (size_t)shot * a.mod_stride;
   float *dat = a.dat + (size_t)shot * a.dat_stride;
-  const size_t o = (size_t)ix * nq + k;
-  float4 ux[9], vx[9];
-#pragma unroll
-  for (int d = 0; d < 9; d++) ux[d] = __ldg(X + o + (long long)(d - 4) * nq);
-  const float4 uzl = __ldg(X + o - 1), uzh = __ldg(X + o + 1);
-  float4 vzl = make_float4(0.f, 0.f, 0.f, 0.f), vzh = vzl;
-  if (ADJ) {
-#pragma unroll
-    for (int d = 0; d < 9; d++) vx[d] = __ldg(V + o + (long long)(d - 4) * nq);
-    vzl = __ldg(V + o - 1);
-    vzh = __ldg(V + o + 1);
-  } else {
-#pragma unroll
-    for (int d = 0; d < 9; d++) vx[d] = vzl;
-    vx[4] = __ldg(V + o);
+  // what no step writes: read before the previous step has ended
+  float4 V, wz, inj;
+  float wx = 0.f;
+  if (f) {
+    V = a.vv[(size_t)ix * nq + k];
+    wz = a.wz[k];
+    wx = a.wx[ix];
+    inj = load_inj<ADJ>(a, mod, dat, f, ix, k, a.it);
   }
-  const float4 inj = load_inj<ADJ>(a, mod, dat, f, ix, k, a.it);
-  quad_out<ADJ>(a, mod, dat, f, ux[4], vx[4], ix, k, a.it);
-  Y[o] = quad_step<ADJ>(a, f, ux, uzl, uzh, vx, vzl, vzh, Y[o], a.wz[k], a.wx[ix], inj, k);
+  pdl_wait();
+  pdl_launch();
+  if (!f) return;
+  const size_t o = (size_t)shot * a.fstride + (size_t)ix * nq + k;
+  const float4 *S = (ADJ ? a.W : a.X) + o;
+  float4 sx9[9];
+#pragma unroll
+  for (int d = 0; d < 9; d++) sx9[d] = S[(d - 4) * nq];
+  const float4 szl = S[-1], szh = S[1];
+  const float4 A = ADJ ? a.X[o] : sx9[4], B = a.Y[o];
+  if (!ADJ && (f & (0xFu << 5)) && a.it + 1 < a.nt) {
+    const float *next = mod + ((long long)(a.it + 1) * a.nx + (ix - a.nb)) * a.nz - a.nb + 4 * k;
+    const int e = __ffs((f >> 5) & 0xFu) - 1;  // the quad's first interior cell
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(next + e));
+  }
+  quad_out<ADJ>(a, mod, dat, f, sx9[4], ix, k, a.it);
+  const float4 r = quad_step<ADJ>(a, f, sx9, szl, szh, A, V, B, wz, wx, inj, k);
+  a.Y[o] = r;
+  if (ADJ) a.Wn[o] = quad_mul(a.one, r, V);
+}
+
+// the adjoint's W of a zero field in both buffers: 0 vv (not a number where
+// the velocity overflows), which the cells outside the stencil keep
+__global__ void zero_w_kernel(const float4 *__restrict__ vv, float4 *__restrict__ W, size_t n,
+                              size_t nfields, float one) {
+  const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n * nfields;
+       i += (size_t)gridDim.x * blockDim.x)
+    W[i] = quad_mul(one, z, vv[i % n]);
 }
 
 // vvpad = (v v) dt^2 on the padded grid, the interior replicated onto every
@@ -406,15 +415,22 @@ __global__ void __launch_bounds__(DOTT) dots_kernel(const float *__restrict__ gg
   if (threadIdx.x < 6) part[(size_t)blockIdx.x * 8 + threadIdx.x] = sh[threadIdx.x][0];
 }
 
-// model side: g.g into slot 6
+// model side: g.g into slot 6.  HBM bound: CGU loads of a thread in flight,
+// added in the order of one by one.
 __global__ void __launch_bounds__(DOTT) sumsq_kernel(const float *__restrict__ g, size_t n,
                                                      double *__restrict__ part) {
   __shared__ double sh[DOTT];
   double s = 0;
-  for (size_t i = (size_t)blockIdx.x * DOTT + threadIdx.x; i < n; i += (size_t)DOTB * DOTT) {
-    const double v = g[i];
-    s = __dadd_rn(s, __dmul_rn(v, v));
+  const size_t step = (size_t)DOTB * DOTT;
+  size_t i = (size_t)blockIdx.x * DOTT + threadIdx.x;
+  for (; i + (CGU - 1) * step < n; i += CGU * step) {
+    float v[CGU];
+#pragma unroll
+    for (int u = 0; u < CGU; u++) v[u] = g[i + u * step];
+#pragma unroll
+    for (int u = 0; u < CGU; u++) s = __dadd_rn(s, __dmul_rn((double)v[u], (double)v[u]));
   }
+  for (; i < n; i += step) s = __dadd_rn(s, __dmul_rn((double)g[i], (double)g[i]));
   sh[threadIdx.x] = s;
   __syncthreads();
   for (int h = DOTT / 2; h > 0; h >>= 1) {
@@ -424,26 +440,53 @@ __global__ void __launch_bounds__(DOTT) sumsq_kernel(const float *__restrict__ g
   if (threadIdx.x == 0) part[(size_t)blockIdx.x * 8 + 6] = sh[0];
 }
 
-__global__ void dots_final_kernel(const double *__restrict__ part, double *__restrict__ out) {
+// all block sums into shared memory at once, then added in block order
+__global__ void __launch_bounds__(DOTT) dots_final_kernel(const double *__restrict__ part,
+                                                          double *__restrict__ out) {
+  __shared__ double sh[DOTB * 8];
+  for (int i = threadIdx.x; i < DOTB * 8; i += DOTT) sh[i] = (i & 7) < 7 ? part[i] : 0.;
+  __syncthreads();
   const int q = threadIdx.x;
   if (q >= 7) return;
   double s = 0;
-  for (int b = 0; b < DOTB; b++) s = __dadd_rn(s, part[(size_t)b * 8 + q]);
+#pragma unroll 8
+  for (int b = 0; b < DOTB; b++) s = __dadd_rn(s, sh[b * 8 + q]);
   out[q] = s;
 }
 
 // np_cgstep's update of one side (wave_cgstep.c:58-66): S = beta S +
-// alfa g (sscal, then saxpy), x += S; forget starts S from zero
-__global__ void cg_update_kernel(float *__restrict__ S, float *__restrict__ x,
-                                 const float *__restrict__ g, size_t n, float alfa, float beta,
-                                 int forget) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    float s = forget ? 0.f : S[i];
-    s = fmul(s, beta);
-    s = fadd(s, fmul(alfa, g[i]));
+// alfa g (sscal, then saxpy), x += S; forget starts S from zero.  HBM bound;
+// CGU elements per thread in flight.
+__device__ __forceinline__ void cg_update1(float &S, float &x, float g, float alfa, float beta) {
+  S = fadd(fmul(S, beta), fmul(alfa, g));
+  x = fadd(x, S);
+}
+__global__ void __launch_bounds__(DOTT) cg_update_kernel(float *__restrict__ S,
+                                                         float *__restrict__ x,
+                                                         const float *__restrict__ g, size_t n,
+                                                         float alfa, float beta, int forget) {
+  const size_t step = (size_t)gridDim.x * DOTT;
+  size_t i = (size_t)blockIdx.x * DOTT + threadIdx.x;
+  for (; i + (CGU - 1) * step < n; i += CGU * step) {
+    float s[CGU], y[CGU], d[CGU];
+#pragma unroll
+    for (int u = 0; u < CGU; u++) {
+      s[u] = forget ? 0.f : S[i + u * step];
+      y[u] = x[i + u * step];
+      d[u] = g[i + u * step];
+    }
+#pragma unroll
+    for (int u = 0; u < CGU; u++) {
+      cg_update1(s[u], y[u], d[u], alfa, beta);
+      S[i + u * step] = s[u];
+      x[i + u * step] = y[u];
+    }
+  }
+  for (; i < n; i += step) {
+    float s = forget ? 0.f : S[i], y = x[i];
+    cg_update1(s, y, g[i], alfa, beta);
     S[i] = s;
-    x[i] = fadd(x[i], s);
+    x[i] = y;
   }
 }
 
@@ -494,14 +537,20 @@ static int check_args(const pw_fwi_args *a, bool need_shots) {
 
 // Resident plan: the largest cluster (16, 8, 4, 2 CTAs, one per SM) whose
 // bands of at least 4 columns fit in shared memory and that the device can
-// schedule; otherwise (or with PW_LSTRI_RESIDENT=0) the step-per-launch path.
-// The adjoint (LapT reads 9 more vv quads per quad) takes the step path
-// where its resident form would need a 16-CTA cluster: on the passive
-// demos' grid (250 x 454 padded, nt 3001) one adjoint application runs
-// 12.4 ms step by step against 15.2 ms resident, while the modelling stays
-// resident (11.7 against 12.4 ms).  PW_LSTRI_RESIDENT=1 keeps every
-// operator resident where it fits.
-static void make_plan(const pw_fwi_args *a, bool adj, Plan &p) {
+// schedule, where it beats a launch per step.  A resident step costs 0.78 us
+// (the cluster barrier) and 1 us per 8000 quads of the padded grid (adjoint:
+// 6000), for as many shots as clusters fit at once; a launched step costs
+// 2.1 us until it fills the chip.  Measured, us per step resident / launched,
+// quads in brackets: one shot [2500] 1.2 / 2.1, [6400] 1.6 / 2.1, [8100]
+// 2.0 / 2.2, [12100] 2.3 / 2.1, [28600] 3.8 / 2.1; adjoint [6400] 1.8 / 2.1,
+// [8100] 2.4 / 2.1, [28600] 5.1 / 2.1; 8 shots, two waves [1600] 1.9 / 2.1,
+// [2500] 2.4 / 2.0, [28600] 7.9 / 4.3.  Several shots that fit in one wave
+// stay one launch at every size, although steps are faster from 10000 quads
+// on ([28600], 2 shots: 3.9 / 2.3): the host thread is free meanwhile.  So do
+// shots whose fields would take more than 256 MB of workspace (or a grid of
+// more than 65535 rows), which the resident form does without.
+// PW_LSTRI_RESIDENT=1 keeps every operator resident where it fits, 0 none.
+static void make_plan(const pw_fwi_args *a, bool adj, int nshots, Plan &p) {
   p.nzp = a->nz + 2 * a->nb;
   p.nxp = a->nx + 2 * a->nb;
   p.nq = (p.nzp + 3) / 4;
@@ -524,8 +573,9 @@ static void make_plan(const pw_fwi_args *a, bool adj, Plan &p) {
     void *fn = adj ? resident_fn<true>(ipt) : resident_fn<false>(ipt);
     static std::mutex mu;
     static std::map<std::pair<int, void *>, size_t> attr_max;
-    static std::map<std::tuple<int, void *, size_t, int>, bool> seen;
+    static std::map<std::tuple<int, void *, size_t, int>, int> seen;  // clusters at once
     bool ok = true;
+    int nclusters = 0;
     {
       std::lock_guard<std::mutex> lock(mu);
       size_t &am = attr_max[std::make_pair(dev, fn)];
@@ -540,7 +590,7 @@ static void make_plan(const pw_fwi_args *a, bool adj, Plan &p) {
       const auto key = std::make_tuple(dev, fn, smem, C);
       const auto hit = seen.find(key);
       if (ok && hit != seen.end()) {
-        ok = hit->second;
+        nclusters = hit->second;
       } else if (ok) {
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
@@ -553,14 +603,17 @@ static void make_plan(const pw_fwi_args *a, bool adj, Plan &p) {
         cfg.dynamicSmemBytes = smem;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        int nclusters = 0;
-        ok = cudaOccupancyMaxActiveClusters(&nclusters, fn, &cfg) == cudaSuccess && nclusters >= 1;
-        seen[key] = ok;
+        if (cudaOccupancyMaxActiveClusters(&nclusters, fn, &cfg) != cudaSuccess) nclusters = 0;
+        seen[key] = nclusters;
       }
+      ok = ok && nclusters >= 1;
       cudaGetLastError();
     }
     if (!ok) continue;
-    if (adj && C == 16 && !force) return;
+    const int waves = (nshots + nclusters - 1) / nclusters;
+    const double res_us = waves * (0.78 + (double)p.nxp * p.nq / (adj ? 6000. : 8000.));
+    const bool room = nshots <= 65535 && (size_t)nshots * p.nxp * p.nq * 32 <= (size_t(256) << 20);
+    if (res_us > 2.1 && (adj || nshots == 1 || (waves > 1 && room)) && !force) return;
     p.resident = true;
     p.C = C;
     p.w = w;
@@ -648,8 +701,8 @@ static int upload_tables(const pw_fwi_args *a, const Plan &p, const Tables &t, c
 }
 
 // One application of the operator to nshots shots (mod / dat strides in
-// Args).  fields: 2 * nshots fields for the step path (unused when
-// resident).  Returns the number of kernel launches through `launches`.
+// Args).  fields: 2 (modelling) or 4 (adjoint) * nshots fields for the step
+// path (unused when resident).  Returns the number of kernel launches through `launches`.
 static int run_op(const Plan &p, Args g, bool adj, int nshots, float4 *fields, cudaStream_t st,
                   long long &launches) {
   if (p.resident) {
@@ -672,15 +725,27 @@ static int run_op(const Plan &p, Args g, bool adj, int nshots, float4 *fields, c
     return PW_OK;
   }
   g.fstride = (size_t)p.nxp * p.nq;
-  float4 *F0 = fields, *F1 = fields + (size_t)nshots * g.fstride;
-  PW_CUDA(cudaMemsetAsync(fields, 0, (size_t)2 * nshots * g.fstride * sizeof(float4), st));
+  g.nqd = make_fast_div(p.nq);
+  const size_t ff = (size_t)nshots * g.fstride;
+  PW_CUDA(cudaMemsetAsync(fields, 0, 2 * ff * sizeof(float4), st));
+  if (adj) {
+    zero_w_kernel<<<148, 256, 0, st>>>(g.vv, fields + 2 * ff, g.fstride, (size_t)2 * nshots, g.one);
+    PW_CUDA(cudaGetLastError());
+  }
   const dim3 grid((unsigned)ceil_div((long long)p.nxp * p.nq, SNTH), (unsigned)nshots);
   for (int s = 0; s < g.nt; s++) {
+    const int x = s & 1;
     g.it = adj ? g.nt - 1 - s : s;
-    g.X = (s & 1) ? F1 : F0;
-    g.Y = (s & 1) ? F0 : F1;
-    if (adj) step_kernel<true><<<grid, SNTH, 0, st>>>(g);
-    else step_kernel<false><<<grid, SNTH, 0, st>>>(g);
+    g.X = fields + x * ff;
+    g.Y = fields + (1 - x) * ff;
+    if (adj) {
+      g.W = fields + (2 + x) * ff;
+      g.Wn = fields + (3 - x) * ff;
+    }
+    // the first step waits for all that came before, as it reads ahead of pdl_wait
+    auto fn = adj ? step_kernel<true> : step_kernel<false>;
+    if (s == 0) fn<<<grid, SNTH, 0, st>>>(g);
+    else PW_CUDA(launch_pdl(fn, grid, dim3(SNTH), 0, st, g));
     PW_CUDA(cudaGetLastError());
     launches += 1;
   }
@@ -713,13 +778,13 @@ extern "C" int pw_timerev(const pw_fwi_args *a, int adj, const float *vel, float
   cudaStream_t st = (cudaStream_t)stream;
   const bool host = (a->flags & PW_HOST_PTRS) != 0;
   Plan p;
-  make_plan(a, adj != 0, p);
+  make_plan(a, adj != 0, 1, p);
   print_plan(adj ? "adjoint" : "modelling", p, 1);
   const size_t nm = (size_t)a->nz * a->nx * a->nt, nd = (size_t)a->nx * a->nt;
   Carve cv;
   Tables t;
   carve_tables(a, p, host, cv, t);
-  const size_t o_f = cv.add(p.resident ? 0 : (size_t)2 * p.nxp * p.nq * sizeof(float4));
+  const size_t o_f = cv.add(p.resident ? 0 : (size_t)(adj ? 4 : 2) * p.nxp * p.nq * sizeof(float4));
   const size_t o_m = cv.add(host ? nm * 4 : 0);
   const size_t o_d = cv.add(host ? nd * 4 : 0);
   Workspace &ws = Workspace::for_current_device();
@@ -760,8 +825,8 @@ extern "C" int pw_lstri_forward(const pw_fwi_args *a, const float *vel, const fl
   cudaStream_t st = (cudaStream_t)stream;
   const bool host = (a->flags & PW_HOST_PTRS) != 0;
   Plan p;
-  make_plan(a, false, p);
   const int ns = a->ns;
+  make_plan(a, false, ns, p);
   print_plan("modelling", p, ns);
   const size_t nm = (size_t)a->nz * a->nx * a->nt, nd = (size_t)a->nx * a->nt;
   Carve cv;
@@ -811,8 +876,8 @@ extern "C" int pw_lstri_invert(const pw_fwi_args *a, const float *vel, const flo
   cudaStream_t st = (cudaStream_t)stream;
   const bool host = (a->flags & PW_HOST_PTRS) != 0;
   Plan pa, pf;
-  make_plan(a, true, pa);
-  make_plan(a, false, pf);
+  make_plan(a, true, 1, pa);
+  make_plan(a, false, 1, pf);
   print_plan("adjoint", pa, 1);
   print_plan("modelling", pf, 1);
   const int ns = a->ns;
@@ -821,7 +886,7 @@ extern "C" int pw_lstri_invert(const pw_fwi_args *a, const float *vel, const flo
   Tables t;
   carve_tables(a, pa, host, cv, t);
   const bool fields = !(pa.resident && pf.resident);
-  const size_t o_f = cv.add(fields ? (size_t)2 * pa.nxp * pa.nq * sizeof(float4) : 0);
+  const size_t o_f = cv.add(fields ? (size_t)4 * pa.nxp * pa.nq * sizeof(float4) : 0);
   const size_t o_x = cv.add(host ? nm * 4 : 0);
   const size_t o_g = cv.add(nm * 4);
   const size_t o_S = cv.add(nm * 4);
@@ -850,7 +915,7 @@ extern "C" int pw_lstri_invert(const pw_fwi_args *a, const float *vel, const flo
   auto reduce = [&](bool model) -> int {
     dots_kernel<<<DOTB, DOTT, 0, st>>>(gg, Ss, rr, nd, part);
     if (model) sumsq_kernel<<<DOTB, DOTT, 0, st>>>(gv, nm, part);
-    dots_final_kernel<<<1, 32, 0, st>>>(part, dots);
+    dots_final_kernel<<<1, DOTT, 0, st>>>(part, dots);
     PW_CUDA(cudaGetLastError());
     launches += model ? 3 : 2;
     PW_CUDA(cudaMemcpyAsync(h, dots, 8 * sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -912,8 +977,8 @@ extern "C" int pw_lstri_invert(const pw_fwi_args *a, const float *vel, const flo
         alfa = (sds * gdr - gds * sdr) / determ;
         beta = (-gds * gdr + gdg * sdr) / determ;
       }
-      cg_update_kernel<<<1184, 256, 0, st>>>(S, x, gv, nm, (float)alfa, (float)beta, forget);
-      cg_update_kernel<<<592, 256, 0, st>>>(Ss, rr, gg, nd, (float)alfa, (float)beta, forget);
+      cg_update_kernel<<<1184, DOTT, 0, st>>>(S, x, gv, nm, (float)alfa, (float)beta, forget);
+      cg_update_kernel<<<592, DOTT, 0, st>>>(Ss, rr, gg, nd, (float)alfa, (float)beta, forget);
       PW_CUDA(cudaGetLastError());
       launches += 2;
     }

@@ -160,3 +160,36 @@ def test_pfwi3d_step_sizes(oracle, cuda_lib, nz, nx, ny, nb, ns):
     g, J = fwi3d.gradient3d(vt, wav, dobs, geom)
     go, Jo = oracle.pf3_gradient_exact(vt, wav, dobs, geom)
     assert rel_l2(g, go) < 1e-4 and abs(J - Jo) < 1e-4 * Jo
+
+
+# both sides of the rule that picks the lstri plan (small and large grids, one wave of shots
+# and more), odd depths, and a velocity whose square overflows: the cluster-resident kernel, a
+# launch per step and the default give identical bits (NaN where the others do)
+@pytest.mark.parametrize("nz,nx,nb,ns,vmax", [(30, 37, 9, 1, 3.0), (85, 90, 40, 1, 3.0),
+                                              (131, 150, 40, 1, 3.0), (131, 150, 40, 2, 3.0),
+                                              (33, 34, 6, 24, 3.0), (70, 83, 20, 24, 3.0),
+                                              (42, 45, 8, 1, 1e25)])
+def test_lstri_plans_agree(cuda_lib, monkeypatch, nz, nx, nb, ns, vmax):
+    from pywave_b200 import lstri
+    nt = 40
+    rng = np.random.default_rng(nz)
+    vel = (1.5 + 1.5 * rng.random((nz, nx))).astype(np.float32)
+    if vmax > 3.0:
+        vel[5, 7] = vel[-1, 3] = vmax
+    par = dict(nz=nz, nx=nx, dz=0.01, dx=0.012, oz=0, ox=0, nt=nt, dt=0.001, ot=0, ns=ns, ds=0.1,
+               os=0.0, nb=nb, coef=0.01, f0=10, acqui_type=1, interval=1, niter=2, rz=2)
+    src = rng.standard_normal((nz, nx, nt, ns)).astype(np.float32)
+    dat = rng.standard_normal((nt, nx)).astype(np.float32)
+    got = []
+    for r in (None, "1", "0"):
+        if r is None:
+            monkeypatch.delenv("PW_LSTRI_RESIDENT", raising=False)
+        else:
+            monkeypatch.setenv("PW_LSTRI_RESIDENT", r)
+        got.append([lstri.lstri_forward(vel, src, par),
+                    lstri.timerev(False, vel, dict(par, ns=1), mod=src[..., 0]),
+                    lstri.timerev(True, vel, dict(par, ns=1), dat=dat)])
+    for other in got[1:]:
+        for x, y in zip(got[0], other):
+            assert np.array_equal(x, y, equal_nan=True)
+    assert all(np.abs(x[np.isfinite(x)]).max() > 0 for x in got[0])
