@@ -91,6 +91,9 @@ struct PfArgs {
   const float *tin;           // ADJ_EXACT: term of the forward step [shot] (field layout)
   long long tin_stride;
   int imaging;                // ADJ_REF: this step images
+  int prev;                   // host: the mode last launched with these arguments.  A step that
+                              // follows one of its own mode overlaps it (its arguments of that
+                              // mode are read ahead); any other waits for all that came before
 };
 
 __device__ __forceinline__ float el(const float4 &v, int e) {
@@ -189,7 +192,11 @@ __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast
 // 8 planes over a shared-memory ring: 626 instructions per float4, now 290);
 // 8 shots of 271 x 421 forward 6.4 us (16.1).  Marching 4 to 16 planes with
 // the 9-deep queue in registers ran 23 to 28 us, two planes per thread 20.7,
-// 8 planes per CTA 21.9, CTAs of consecutive lanes only 21.4.
+// 8 planes per CTA 21.9, CTAs of consecutive lanes only 21.4.  A small survey
+// (4 shots of 140 x 201) is bound by the latency of dependent launches: with
+// all that no step of the mode writes read (and the imaging's division done)
+// before the previous step has ended, forward and reference adjoint take 3.4
+// us on average, 3.9 with all reads after it.
 template <int MODE, bool PAS>
 __global__ void __launch_bounds__(32 * PF_XW, MODE == ADJ_REF || PAS ? 5 : 6)
     pf_step_kernel(const __grid_constant__ PfArgs a) {
@@ -199,62 +206,80 @@ __global__ void __launch_bounds__(32 * PF_XW, MODE == ADJ_REF || PAS ? 5 : 6)
   const int z4 = (int)item - chunk * a.nz4.d;
   const int x = chunk * PF_XW + (threadIdx.x >> 5);
   const int iz0 = 4 * z4;
-  pdl_sync();
-  if (x >= a.pnx) return;
+  const bool live = x < a.pnx;
   const long long lz = a.lz;
   const long long o0 = pfoff(a.lz, iz0, x);  // own float4
   const float *pc = a.cur + s * a.fstep + o0;
   float *pn = a.nxt + s * a.fstep + o0;
-  const float *pv = a.V + o0;
-  const float *pt = MODE == ADJ_EXACT ? a.tin + s * a.tin_stride + o0 : nullptr;
   float *pg = MODE == ADJ_EXACT ? a.grad + s * a.gstride + o0 : nullptr;
   float *po = (MODE == FWD && a.tout) ? a.tout + s * a.tout_stride + o0 : nullptr;
   float *const gs = MODE == ADJ_REF ? a.grad + s * a.gstride : nullptr;
-
-  float4 q[9];  // own column, planes x-4 .. x+4
-#pragma unroll
-  for (int d = 0; d < 9; d++) q[d] = ld4(pc + (d - 4) * lz);
-  const float4 c = q[4], L = ld4(pc - 4), R = ld4(pc + 4), p4 = ld4(pn), V4 = ld4(pv);
-  float4 tf = make_float4(0.f, 0.f, 0.f, 0.f), g4 = tf;
-  if (MODE == ADJ_EXACT) {
-    tf = __ldcs(reinterpret_cast<const float4 *>(pt));
-    g4 = ld4(pg);
-  }
-  const float bxf = a.bx[x];
-  const float4 bz4 = ld4(a.bz + iz0);
-  // the stencil's rows [4, pnz - 4): the first and the last float4 of a column
-  // hold none, at most one float4 holds some of both
-  const bool lz_any = z4 >= 1 && iz0 < a.pnz - 4;
-  const bool lz_full = lz_any && iz0 + 3 < a.pnz - 4;
-  const bool rec_row = a.rz >= iz0 && a.rz < iz0 + 4;
-  const bool src_z = MODE == FWD && !PAS && iz0 <= a.src_z1 && iz0 + 3 >= a.src_z0;
   const ShotGeo &sg = a.geo[s];
-  const f2 k1 = pk2(a.one, a.one);
-  const f2 kc[5] = {pk2(a.c0, a.c0), pk2(a.c1, a.c1), pk2(a.c2, a.c2), pk2(a.c3, a.c3),
-                    pk2(a.c4, a.c4)};
-
-  // ADJ_REF imaging operands of this plane
-  double rw[4];
-  float rt[4], rg[4];
+  const bool rec_row = a.rz >= iz0 && a.rz < iz0 + 4;
   const bool xin = x >= a.nb && x < a.nb + a.nx;
   const bool img = MODE == ADJ_REF && a.imaging && xin;
+
+  // what no step of this mode writes, read before the previous step has ended
+  float4 V4 = make_float4(0.f, 0.f, 0.f, 0.f), bz4 = V4, tf = V4, g4 = V4;
+  float bxf = 0.f, resid = 0.f;
+  int rir = -1;
+  double rw[4];  // ADJ_REF imaging operands
+  float rt[4], rg[4];
+  if (live) {
+    V4 = ld4(a.V + o0);
+    bz4 = ld4(a.bz + iz0);
+    bxf = a.bx[x];
+    if (MODE == ADJ_EXACT)
+      tf = __ldcs(reinterpret_cast<const float4 *>(a.tin + s * a.tin_stride + o0));
+    if (rec_row) {
+      const int d = x - sg.r0v;
+      if (d >= 0) {
+        const int ir = a.drv == 1 ? d : (d % a.drv == 0 ? d / a.drv : -1);
+        if (ir >= 0 && ir < sg.nr2) rir = sg.r02 + ir;
+      }
+      if (MODE != FWD && rir >= 0) resid = a.res[((size_t)s * a.nt + a.it) * a.nr + rir];
+    }
+  }
   if (MODE == ADJ_REF) {
 #pragma unroll
     for (int e = 0; e < 4; e++) {
       const int iz = iz0 + e;
       rw[e] = 0.;
-      rt[e] = rg[e] = 0.f;
+      rt[e] = 0.f;
       if (img && iz >= a.nb && iz < a.nb + a.nz) {
         const size_t k = (size_t)(x - a.nb) * a.nz + (iz - a.nb);
         const size_t ks = s * a.wstride + k;
-        // wave[wit+1] - 2.*wave[wit] + wave[wit-1] in double, left to right
+        // (wave[wit+1] - 2.*wave[wit] + wave[wit-1]) / wdt2 in double, left to right
         rw[e] = __dadd_rn(__dsub_rn((double)a.wnext[ks], __dmul_rn(2., (double)a.wcur[ks])),
                           (double)a.wprev[ks]);
+        rw[e] = __ddiv_rn(rw[e], (double)a.wdt2);
         rt[e] = a.m2v3[k];
-        rg[e] = gs[k];
       }
     }
   }
+  pdl_sync();
+  if (!live) return;
+
+  float4 q[9];  // own column, planes x-4 .. x+4
+#pragma unroll
+  for (int d = 0; d < 9; d++) q[d] = ld4(pc + (d - 4) * lz);
+  const float4 c = q[4], L = ld4(pc - 4), R = ld4(pc + 4), p4 = ld4(pn);
+  if (MODE == ADJ_EXACT) g4 = ld4(pg);
+  if (MODE == ADJ_REF) {
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      const int iz = iz0 + e;
+      rg[e] = img && iz >= a.nb && iz < a.nb + a.nz ? gs[(size_t)(x - a.nb) * a.nz + (iz - a.nb)] : 0.f;
+    }
+  }
+  // the stencil's rows [4, pnz - 4): the first and the last float4 of a column
+  // hold none, at most one float4 holds some of both
+  const bool lz_any = z4 >= 1 && iz0 < a.pnz - 4;
+  const bool lz_full = lz_any && iz0 + 3 < a.pnz - 4;
+  const bool src_z = MODE == FWD && !PAS && iz0 <= a.src_z1 && iz0 + 3 >= a.src_z0;
+  const f2 k1 = pk2(a.one, a.one);
+  const f2 kc[5] = {pk2(a.c0, a.c0), pk2(a.c1, a.c1), pk2(a.c2, a.c2), pk2(a.c3, a.c3),
+                    pk2(a.c4, a.c4)};
   float dv[4] = {0.f, 0.f, 0.f, 0.f};
   if (MODE == FWD && PAS) {
     // the interior cells' source samples
@@ -267,16 +292,8 @@ __global__ void __launch_bounds__(32 * PF_XW, MODE == ADJ_REF || PAS ? 5 : 6)
     }
   }
   // receivers read the field before the update (wave_fwimodeling.c:76-79)
-  int rir = -1;
-  if (rec_row) {
-    const int d = x - sg.r0v;
-    if (d >= 0) {
-      const int ir = a.drv == 1 ? d : (d % a.drv == 0 ? d / a.drv : -1);
-      if (ir >= 0 && ir < sg.nr2) rir = sg.r02 + ir;
-    }
-    if (MODE == FWD && rir >= 0 && a.rec)
-      a.rec[((size_t)s * a.nt + a.it) * a.nr + rir] = el(c, a.rz - iz0);
-  }
+  if (MODE == FWD && rir >= 0 && a.rec)
+    a.rec[((size_t)s * a.nt + a.it) * a.nr + rir] = el(c, a.rz - iz0);
   if (MODE == FWD && a.snap && xin) {
 #pragma unroll
     for (int e = 0; e < 4; e++) {
@@ -342,10 +359,9 @@ __global__ void __launch_bounds__(32 * PF_XW, MODE == ADJ_REF || PAS ? 5 : 6)
             set_el(term4, e, fadd(el(term4, e), fmul(sg.sw[k], w)));
     }
   } else if (rir >= 0) {
-    const float r = a.res[((size_t)s * a.nt + a.it) * a.nr + rir];
 #pragma unroll
     for (int e = 0; e < 4; e++)
-      if (iz0 + e == a.rz) set_el(term4, e, fadd(el(term4, e), r));
+      if (iz0 + e == a.rz) set_el(term4, e, fadd(el(term4, e), resid));
   }
   {
     // b = S(a_{k-1} as stored): z faces then x faces (apply_sponge);
@@ -380,9 +396,7 @@ __global__ void __launch_bounds__(32 * PF_XW, MODE == ADJ_REF || PAS ? 5 : 6)
       const int iz = iz0 + e;
       if (iz >= a.nb && iz < a.nb + a.nz) {
         const size_t k = (size_t)(x - a.nb) * a.nz + (iz - a.nb);
-        const double gsum = __dmul_rn(__dmul_rn(__ddiv_rn(rw[e], (double)a.wdt2),
-                                                (double)el(c, e)),
-                                      (double)rt[e]);
+        const double gsum = __dmul_rn(__dmul_rn(rw[e], (double)el(c, e)), (double)rt[e]);
         gs[k] = __double2float_rn(__dadd_rn((double)rg[e], gsum));
       }
     }
@@ -953,10 +967,16 @@ static int setup(const pw_fwi_args *a, Setup &S, bool passive = false) {
 }
 
 template <int MODE, bool PAS = false>
-static int launch_one(const Setup &S, const PfArgs &p, int nshots, cudaStream_t st) {
+static int launch_one(const Setup &S, PfArgs &p, int nshots, cudaStream_t st) {
   const long long lanes = (long long)p.nz4.d * ceil_div(S.pnx, PF_XW);
   const dim3 grid((unsigned)ceil_div(lanes, 32), (unsigned)nshots);
-  PW_CUDA(launch_pdl(pf_step_kernel<MODE, PAS>, grid, dim3(32 * PF_XW), 0, st, p));
+  if (p.prev == MODE) {
+    PW_CUDA(launch_pdl(pf_step_kernel<MODE, PAS>, grid, dim3(32 * PF_XW), 0, st, p));
+  } else {
+    pf_step_kernel<MODE, PAS><<<grid, 32 * PF_XW, 0, st>>>(p);
+    PW_CUDA(cudaGetLastError());
+  }
+  p.prev = MODE;
   return PW_OK;
 }
 
@@ -970,6 +990,7 @@ static int launch(const Setup &S, PfArgs &p, int mode, int nshots, cudaStream_t 
 
 static void base_args(const Setup &S, PfArgs &p) {
   memset(&p, 0, sizeof p);
+  p.prev = -1;
   p.pnz = S.pnz;
   p.pnx = S.pnx;
   p.lz = S.lz;
