@@ -200,7 +200,7 @@ __device__ __forceinline__ float4 taper_quad(const float4 &v, const float (&wz)[
 // march y through shared-memory rings; 2-D columns marched through a
 // per-thread ring): 261^3, 4 groups 231 -> 215 us (183 instructions per
 // float4 instead of 263); 261^3 forward 103 -> 56; 141^3 forward 25 -> 9.6;
-// 561 x 1561 forward 8.2 -> 3.6; 12 uneven shots 44.7 -> 29.  Marching up to 8
+// 561 x 1561 forward 8.2 -> 3.6; 12 uneven shots 44.7 -> 27.4.  Marching up to 8
 // planes per thread with the y neighbours in registers: 217 / 77 / 13 us on
 // the 3-D grids; CTAs of 4 x 4 columns 250 / 84 / 12.8, of 8 slots x 4 x 4
 // 226 / 67 / 10.9; the groups of a launch in separate CTAs 242.
@@ -217,8 +217,9 @@ __device__ __forceinline__ void square_into(float4 &prod, const float4 &u) {
 }
 
 // Groups [g0, g1) of one float4; the square product of their new values in
-// group order multiplies `prod` (imaging steps).
-template <bool XT, bool TRI, bool SNAP>
+// group order multiplies `prod` (imaging steps).  EARLY: what no step writes
+// is read before the previous step has ended (else the kernel waits first).
+template <bool XT, bool TRI, bool SNAP, bool EARLY>
 __device__ __forceinline__ void quad_update(const StepArgs &a, int slot, int ix, int y, int it,
                                             bool swap, int g0, int g1, float4 &prod,
                                             float4 *last = nullptr) {
@@ -252,6 +253,10 @@ __device__ __forceinline__ void quad_update(const StepArgs &a, int slot, int ix,
     }
   }
   const bool in_xy = SNAP && ix >= a.nbx && ix < a.nbx + a.nx1 && y >= a.nby && y < a.nby + a.ny1;
+  if (EARLY) {  // so far only what no step writes: the previous step may still run
+    pdl_wait();
+    pdl_launch();
+  }
 #pragma unroll 1
   for (int gi = TRI ? g0 : 0; gi < (TRI ? g1 : 1); gi++) {
     const float *A = (swap ? a.nxt[gi] : a.cur[gi]) + o;
@@ -371,40 +376,44 @@ __device__ __forceinline__ void quad_stats(const StepArgs &a, bool live, int slo
 }
 
 // 3-D: QXW columns of one plane per CTA
-template <bool TRI, bool SNAP>
+template <bool TRI, bool SNAP, bool EARLY>
 __global__ void __launch_bounds__(32 * QXW, 6)
     quad3_kernel(const __grid_constant__ StepArgs a) {
   int group;
   const int slot = quad_slot(a, blockIdx.x, group);
   const int ix = group * QXW + (threadIdx.x >> 5);
-  pdl_wait();
-  pdl_launch();
+  if (!EARLY) {
+    pdl_wait();
+    pdl_launch();
+  }
   // a launch has at most 65535 block rows: further planes along blockIdx.z
   const int y = zigzag(a.it & a.zig, blockIdx.z * gridDim.y + blockIdx.y, gridDim.y * gridDim.z);
   const bool live = ix < a.g.nx && y < a.g.ny;
   if (a.stats != nullptr) quad_stats<TRI>(a, live, slot, ix, y);
   if (!live) return;
   float4 prod = make_float4(1.f, 1.f, 1.f, 1.f);
-  quad_update<true, TRI, SNAP>(a, slot, ix, y, a.it, false, 0, a.ngroups, prod);
+  quad_update<true, TRI, SNAP, EARLY>(a, slot, ix, y, a.it, false, 0, a.ngroups, prod);
   if (SNAP && TRI) quad_image(a, slot, ix, y, prod);
 }
 
 // 2-D: QW2 columns of the kernel's y (the model's x) per CTA, and one warp per
 // column and group (a 2-D step is a chain of load latencies: the groups in
 // turn in one thread took 4.8 us per step of 261^2 and 4 groups, in warps of
-// their own 2D4G).  The image product meets the groups in shared memory.
-template <bool TRI, bool SNAP>
+// their own 3.0, with the fixed operands read early 2.4).  The image product meets the groups in shared memory.
+template <bool TRI, bool SNAP, bool EARLY>
 __global__ void __launch_bounds__(32 * QW2 * (TRI ? MAXG : 1))
     quad2_kernel(const __grid_constant__ StepArgs a) {
   __shared__ float4 fac[SNAP && TRI ? 32 * QW2 * MAXG : 1];
   int group;
   const int slot = quad_slot(a, zigzag(a.it & a.zig, blockIdx.x, gridDim.x), group);
   const int w = threadIdx.x >> 5, gi = TRI ? w / QW2 : 0, y = group * QW2 + (TRI ? w % QW2 : w);
-  pdl_wait();
-  pdl_launch();
+  if (!EARLY) {
+    pdl_wait();
+    pdl_launch();
+  }
   const bool live = y < a.g.ny;
   float4 prod = make_float4(1.f, 1.f, 1.f, 1.f), u;
-  if (live) quad_update<false, TRI, SNAP>(a, slot, 0, y, a.it, false, gi, gi + 1, prod, &u);
+  if (live) quad_update<false, TRI, SNAP, EARLY>(a, slot, 0, y, a.it, false, gi, gi + 1, prod, &u);
   if (SNAP && TRI) {
     fac[threadIdx.x] = u;
     __syncthreads();
@@ -707,9 +716,7 @@ __global__ void __launch_bounds__(32 * QW2) batch_kernel(const StepArgs *args, c
   if constexpr (TAB) {
     const StepArgs &sa = reinterpret_cast<const StepArgs *>(batch_tab)[item.x];
     const int slot = quad_slot(sa, item.y, group), y = group * QW2 + (threadIdx.x >> 5);
-    pdl_wait();
-    pdl_launch();
-    if (y < sa.g.ny) quad_update<false, false, false>(sa, slot, 0, y, it, (it & 1) != 0, 0, 1, none);
+    if (y < sa.g.ny) quad_update<false, false, false, true>(sa, slot, 0, y, it, (it & 1) != 0, 0, 1, none);
   } else {
     __shared__ StepArgs sa;
     const int *src = reinterpret_cast<const int *>(args + item.x);
@@ -718,9 +725,7 @@ __global__ void __launch_bounds__(32 * QW2) batch_kernel(const StepArgs *args, c
       dst[i] = src[i];
     __syncthreads();
     const int slot = quad_slot(sa, item.y, group), y = group * QW2 + (threadIdx.x >> 5);
-    pdl_wait();
-    pdl_launch();
-    if (y < sa.g.ny) quad_update<false, false, false>(sa, slot, 0, y, it, (it & 1) != 0, 0, 1, none);
+    if (y < sa.g.ny) quad_update<false, false, false, true>(sa, slot, 0, y, it, (it & 1) != 0, 0, 1, none);
   }
 }
 
@@ -1511,27 +1516,35 @@ struct Plan {
   int S, nzc, WZ, WX;
 };
 
-template <bool TWO_D>
-static void *quad_fn(bool tri, bool snap) {
-  if (TWO_D) {
-    if (tri) return snap ? (void *)quad2_kernel<true, true> : (void *)quad2_kernel<true, false>;
-    return snap ? (void *)quad2_kernel<false, true> : (void *)quad2_kernel<false, false>;
-  }
-  if (tri) return snap ? (void *)quad3_kernel<true, true> : (void *)quad3_kernel<true, false>;
-  return snap ? (void *)quad3_kernel<false, true> : (void *)quad3_kernel<false, false>;
+// The step kernel reads the velocity, the tapers and the samples before the
+// previous step has ended (EARLY) up to this many threads per launch, about a
+// wave at the 2-D kernels' occupancy.  Measured, us per step without / with:
+// 2-D time reversal 69 000 threads 3.00 / 2.44, 168 000 3.90 / 4.05, 620 000
+// 9.2 / 10.1; 2-D forward 30 000 2.31 / 2.18, 150 000 3.38 / 2.99, 220 000
+// 3.57 / 3.85, 1.2 M 11.8 / 11.5, 4 M 42.8 / 44.6; 3-D forward 138 000 3.45 /
+// 3.23, 715 000 9.34 / 9.54, 4.5 M 56.1 / 60.2.  Batches, whose items are read
+// through a table, gain at every size: 12 of 200 x 300 3.68 / 3.17, 12 uneven
+// ones of up to 800 x 1700 28.8 / 27.4.
+constexpr long long EARLY_THREADS = 160000;
+
+template <bool TRI, bool SNAP>
+static void *quad_fn(bool two_d, bool early) {
+  if (two_d) return early ? (void *)quad2_kernel<TRI, SNAP, true> : (void *)quad2_kernel<TRI, SNAP, false>;
+  return early ? (void *)quad3_kernel<TRI, SNAP, true> : (void *)quad3_kernel<TRI, SNAP, false>;
 }
 
 static void plan_quad(bool tri, int G, Plan &p) {
   const Geo &g = p.g;
   const bool two_d = p.dim == 2;
   p.quad = true;
-  p.fn = two_d ? quad_fn<true>(tri, false) : quad_fn<false>(tri, false);
-  p.fn_snap = two_d ? quad_fn<true>(tri, true) : quad_fn<false>(tri, true);
   const long long lanes = (long long)p.nq.d * (two_d ? ceil_div(g.ny, QW2) : ceil_div(g.nx, QXW));
   p.grid = dim3((unsigned)ceil_div(lanes, 32), two_d ? 1u : (unsigned)std::min(g.ny, 65535),
                 two_d ? 1u : (unsigned)ceil_div(g.ny, 65535));
   p.threads = 32 * (two_d ? QW2 * (tri ? G : 1) : QXW);
   p.smem = 0;
+  const bool early = (long long)p.grid.x * p.grid.y * p.grid.z * p.threads <= EARLY_THREADS;
+  p.fn = tri ? quad_fn<true, false>(two_d, early) : quad_fn<false, false>(two_d, early);
+  p.fn_snap = tri ? quad_fn<true, true>(two_d, early) : quad_fn<false, true>(two_d, early);
   if (getenv("PW_AFD_VERBOSE"))
     fprintf(stderr, "afd quad plan: G=%d nq=%d threads=%d grid=%ux%u\n", G, p.nq.d, p.threads,
             p.grid.x, p.grid.y);
@@ -1956,8 +1969,10 @@ static void source_box(StepArgs &s) {
 }
 
 // One step; the quad kernels may overlap their start with the step before.
-static cudaError_t launch_step(void *fn, const Plan &p, void **args, cudaStream_t st) {
-  if (!p.quad) return cudaLaunchKernel(fn, p.grid, dim3(p.threads), args, p.smem, st);
+// The first step waits for all that came before it, as the quad kernels read
+// the velocity, the tapers and the samples ahead of pdl_wait
+static cudaError_t launch_step(void *fn, const Plan &p, bool first, void **args, cudaStream_t st) {
+  if (!p.quad || first) return cudaLaunchKernel(fn, p.grid, dim3(p.threads), args, p.smem, st);
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -2260,7 +2275,7 @@ static int run(const pw_afd_args *a, int G, const int *group, const float *vel, 
     s.img = (img_step && p.quad) ? img : nullptr;
     void *args[] = {(void *)&s, (void *)&maps[k & 1]};
     void *f = (s.wfd || s.img) ? p.fn_snap : fn;
-    PW_CUDA(launch_step(f, p, args, st));
+    PW_CUDA(launch_step(f, p, k == 0, args, st));
     if (img_step && !p.quad) {
       for (int i = 0; i < G; i++) ia.u[i] = B[i];
       image_kernel<<<1184, 256, 0, st>>>(ia);
@@ -2827,7 +2842,7 @@ static int run_noalloc(const pw_afd_args *a, const float *vel, const float *src,
     s.wfd = (snap && wfd) ? wfd + (size_t)(it / a->jsnap) * nvel : nullptr;
     void *args[] = {(void *)&s};
     void *f = s.wfd ? p.fn_snap : fn;
-    PW_CUDA(launch_step(f, p, args, st));
+    PW_CUDA(launch_step(f, p, it == 0, args, st));
     std::swap(A, B);
   }
   if (dat) {

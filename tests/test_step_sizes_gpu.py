@@ -193,3 +193,27 @@ def test_lstri_plans_agree(cuda_lib, monkeypatch, nz, nx, nb, ns, vmax):
         for x, y in zip(got[0], other):
             assert np.array_equal(x, y, equal_nan=True)
     assert all(np.abs(x[np.isfinite(x)]).max() > 0 for x in got[0])
+
+
+# launches below and above the size up to which a step's fixed operands are read before the
+# previous step has ended (160 000 threads): 2-D and 3-D, forward and time reversal
+@pytest.mark.parametrize("shape", [(391, 800), (415, 1650), (60, 40, 31), (92, 70, 61)])
+def test_afd_fixed_operands_read_ahead(oracle, cuda_lib, monkeypatch, shape):
+    import pywave_b200 as pw
+    monkeypatch.setenv("PW_AFD_RESIDENT", "0")
+    nt, dim, nbt = 9, len(shape), 6
+    rng = np.random.default_rng(shape[1])
+    vel = (1500 + 1500 * rng.random(shape)).astype(np.float32)
+    kw = dict(nt=nt, dt=0.001, ax=[0, 10, shape[1]], az=[0, 10, shape[0]], nbt=nbt, ct=0.02, jsnap=4)
+    src = dict(sx=[shape[1] // 2], sz=[0], f=[30.0], t=[0.003], A=[2.0])
+    if dim == 3:
+        kw["ay"] = [0, 10, shape[2]]
+        src["sy"] = [shape[2] // 2]
+    run = pw.afd2d if dim == 2 else pw.afd3d
+    d, w = run(vel, ns=1, **src, **kw)
+    do, wo = oracle.afd(vel, nt, 0.001, (10.0,) * dim, nbt=nbt, ct=0.02, src=src, jsnap=4)
+    assert np.abs(do).max() > 0 and np.array_equal(d, do) and np.array_equal(w, wo)
+    tr = rng.standard_normal((nt,) + shape[1:]).astype(np.float32)
+    _, w = run(vel, dat=tr, tri=True, **kw)
+    _, wo = oracle.afd(vel, nt, 0.001, (10.0,) * dim, nbt=nbt, ct=0.02, tri=True, dat=tr, jsnap=4)
+    assert np.abs(wo).max() > 0 and np.array_equal(w, wo)
