@@ -806,7 +806,7 @@ def run_batch2d(args, world, rank, local):
             "e2e": e2e, "gpu_launches": launches,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": None,
-                         "kernel": "batch_kernel (2-D march, all running shots)",
+                         "kernel": "batch_kernel (all running shots)",
                          "loop_ms": loop_ms, "alg_bytes_per_step": cells * 16,
                          "peak_source": peak_kind},
             "cpu_baseline": cpu, "clocks": clocks}), flush=True)
@@ -934,7 +934,7 @@ def run_c1(args, world, rank, local):
     ms_b = max_over_ranks(e0.elapsed_time(e1), world)
     value = job_rate(pts, args.steps, world, ms_b) / 1e9
     kernel = ("resident_kernel (one cluster launch for all steps, fields in shared memory)"
-              if step_launches == 1 else "march_kernel<TWO_D> (one launch per step)")
+              if step_launches == 1 else "quad2_kernel (one launch per step)")
     e2e = None
     if not args.no_e2e:
         pw.afd2d(vel, **kw)
@@ -1156,7 +1156,7 @@ def run_afd3d(args, world, rank, local):
             "e2e": e2e, "gpu_launches": launches,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": None,
-                         "kernel": "tile_kernel<forward> (one launch per step)",
+                         "kernel": "quad3_kernel<forward> (one launch per step)",
                          "kernel_ms": kern_ms, "alg_bytes_per_launch": alg,
                          "peak_source": peak_kind},
             "cpu_baseline": cpu, "clocks": clocks}), flush=True)
@@ -1435,18 +1435,13 @@ def run_lstri(args, world, rank, local):
     clocks = clk.stop()
     ms = max_over_ranks(e0.elapsed_time(e1), world)
     updates = pad * nt * 2 * niter * LS_NS  # adjoint + modelling per iteration
-    # one modelling operator alone, timed on the device (resident launch)
+    # one modelling operator alone, timed on the device
     fwd_ms = []
     scratch = torch.empty_like(d_d[0])
     for _ in range(3):
         lstri.timerev_torch(False, v_d, dict(par, ns=1), inv_d[0], scratch)
         fwd_ms.append(L.last_timing()[0])
     op_ms = statistics.median(fwd_ms)
-    # fp32 issue bound of one 16-SM cluster: 40 float operations per cell
-    # (Laplacian 30, update 3, two sponge products, injection 2)
-    sm_clk = (clocks or {}).get("sm_mhz") or 1965.0
-    cluster_flops = 16 * 128 * sm_clk * 1e6
-    op_flops = 40.0 * pad * nt
     # end to end through the drop-in module: host data in, host source field out
     e2e = None
     if not args.no_e2e:
@@ -1480,11 +1475,10 @@ def run_lstri(args, world, rank, local):
             "roofline": {"bound": "hbm", "achieved": src_bytes / (op_ms / 1e3) / 1e9,
                          "peak": peak, "unit": "GB/s",
                          "frac": src_bytes / (op_ms / 1e3) / 1e9 / peak, "traffic": None,
-                         "kernel": "tr::resident_kernel modelling (one shot, one launch)",
+                         "kernel": "tr::step_kernel modelling (one shot, one launch per step)",
                          "op_ms": op_ms, "peak_source": peak_kind,
-                         "cluster_fp32_frac": op_flops / (op_ms / 1e3) / cluster_flops,
-                         "note": "one 16-SM cluster per shot: bound by that cluster's fp32 "
-                                 "issue and its per-step barrier, not by HBM"},
+                         "us_per_step": op_ms * 1e3 / nt,
+                         "note": "bound by the latency of dependent launches, not by HBM"},
             "e2e": e2e, "cpu_baseline": cpu, "clocks": clocks}), flush=True)
 
 
@@ -1992,7 +1986,7 @@ def main():
                          "frac": achieved / peak, "traffic": traffic,
                          "traffic_source": "stored ncu figure (profiles/traffic.json), "
                                            "not measured in this run",
-                         "kernel": f"tile_kernel<TRI> x{G} groups + image_kernel every 4th step",
+                         "kernel": f"quad3_kernel<TRI> x{G} groups, the image in every 4th step",
                          "kernel_ms": kern_ms, "alg_bytes_per_launch": alg_bytes,
                          "peak_source": peak_kind},
             "cpu_baseline": cpu,

@@ -14,7 +14,7 @@
 // float4 of 4 consecutive z cells.  Halo cells are never written and stay
 // zero: that is the reference's zero border beyond the expanded grid.
 //
-// Kernels.  2-D runs that fit a thread-block cluster's shared memory take
+// Kernels.  Small 2-D runs that fit a thread-block cluster's shared memory take
 // resident_kernel (every step in one launch); the other 2-D runs and all 3-D
 // runs take the quad kernels, one float4 of z cells per thread and step.  The
 // warp-tile kernels, which march 3-D patches along y through shared-memory

@@ -188,7 +188,7 @@ __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast
 // planes of the group, whose 9-plane columns overlap in L1.
 // Bound: instruction issue and L1 / L2 latency (a 16-shot field pair of 420 x
 // 720 sits in L2).  Measured, one launch: 16 shots of 420 x 720, forward and
-// exact adjoint together 20.2 us on average (39.5 with the former x march of
+// exact adjoint together 20.3 us on average (39.5 with the former x march of
 // 8 planes over a shared-memory ring: 626 instructions per float4, now 290);
 // 8 shots of 271 x 421 forward 6.4 us (16.1).  Marching 4 to 16 planes with
 // the 9-deep queue in registers ran 23 to 28 us, two planes per thread 20.7,
