@@ -46,9 +46,11 @@ enum Mode { FWD = 0, ADJ_REF = 1, ADJ_EXACT = 2 };
 // of x in one binade; scaling x by 2^k scales every step exactly while the
 // intermediate values stay normal, which |x| in [xmin, xmax] ensures.
 // Below xmin (the tiny values at the edge of a wavefield) and above xmax, or
-// when the check fails: div_f64; for NaN or infinity: __fdiv_rn.
+// when the check fails: div_f64; for NaN or infinity, or a divisor that is not
+// finite and positive (the square of a spacing over- or underflows): __fdiv_rn.
 struct DivC {
   float d, zh, zl, xmin, xmax;  // xmin > xmax: no numerator takes the method
+  int f64;                      // 1: d is finite and positive, div_f64 applies
   double dd, rd;                // d and RN(1/d)
 };
 
@@ -118,7 +120,7 @@ __device__ __forceinline__ float min3abs(float a, float b, float c) {
   return r;
 }
 
-// v / d rounded once, through FP64: q = v * RN(1/d) corrected by its exact
+// v / d rounded once, through FP64, for finite d > 0: q = v * RN(1/d) corrected by its exact
 // remainder is v / d to within a rounding of 53 bits, and equals it where
 // v / d has at most 53 bits; a quotient of two floats that is no tie of the
 // float grid (subnormal or not) lies at least 2^-48 of itself from every
@@ -134,8 +136,9 @@ __device__ __forceinline__ float div_f64(float v, double d, double rd) {
 // method, two values per op.  All zero (ahead of the numerical wavefront):
 // zero.  Otherwise (the shell of tiny values around that zone, which crosses
 // most columns while a wave expands) through FP64, or by __fdiv_rn where a
-// numerator is infinite or NaN.  The first test is 8 three-operand minima and
-// maxima for the 8 numerators.
+// numerator is infinite or NaN or a divisor is not finite and positive (x / inf
+// is 0 and 0 / 0 NaN, which the other forms do not give).  The first test is 8
+// three-operand minima and maxima for the 8 numerators.
 // The sign of a zero quotient is not kept (these forms can give +0 for -0):
 // no output depends on it.  The sum of the quotients is then +0 where it
 // should be -0 only if both numerators are -0, for which the centre value c
@@ -157,10 +160,11 @@ __device__ __forceinline__ void div4_sum(const f2 (&tx)[2], const f2 (&tz)[2], c
       t[h] = add2(fma2(tx[h], xh, mul2(tx[h], xl)), fma2(tz[h], zh, mul2(tz[h], zl)));
     return;
   }
+  const bool f64 = cx.f64 && cz.f64;
   t[0] = t[1] = 0ull;
-  if (mx == 0.f) return;
+  if (f64 && mx == 0.f) return;
   float4 r;
-  if (mx <= FLT_MAX) {
+  if (f64 && mx <= FLT_MAX) {
 #pragma unroll
     for (int e = 0; e < 4; e++)
       set_el(r, e, fadd(div_f64(el(x, e), cx.dd, cx.rd), div_f64(el(z, e), cz.dd, cz.rd)));
@@ -830,7 +834,8 @@ static int prepare_div(float d, DivC &c) {
   c.zh = c.zl = 0.f;
   c.xmin = 1.f;
   c.xmax = 0.f;
-  if (d > 0.f && std::isfinite(d)) {
+  c.f64 = d > 0.f && std::isfinite(d);
+  if (c.f64) {
     // zh: the float nearest 1/d (float x float products are exact in double,
     // and 1 - zh*d is exact by Sterbenz's lemma)
     const float z0 = (float)(1.0 / (double)d);
