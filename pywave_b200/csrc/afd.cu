@@ -705,7 +705,8 @@ __global__ void __launch_bounds__(RES_NTH) resident_kernel(const __grid_constant
 // memory first.  The table is written and read under the device's workspace
 // lock only.
 constexpr int BATCH_TAB = 96;
-__constant__ char batch_tab[BATCH_TAB * sizeof(StepArgs)];
+__constant__ StepArgs batch_tab[BATCH_TAB];
+static_assert(sizeof batch_tab <= 65536, "constant memory holds 64 KB");
 
 template <bool TAB>
 __global__ void __launch_bounds__(32 * QW2) batch_kernel(const StepArgs *args, const int2 *items,
@@ -714,7 +715,7 @@ __global__ void __launch_bounds__(32 * QW2) batch_kernel(const StepArgs *args, c
   float4 none;
   int group;
   if constexpr (TAB) {
-    const StepArgs &sa = reinterpret_cast<const StepArgs *>(batch_tab)[item.x];
+    const StepArgs &sa = batch_tab[item.x];
     const int slot = quad_slot(sa, item.y, group), y = group * QW2 + (threadIdx.x >> 5);
     if (y < sa.g.ny) quad_update<false, false, false, true>(sa, slot, 0, y, it, (it & 1) != 0, 0, 1, none);
   } else {
