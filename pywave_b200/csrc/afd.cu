@@ -2688,8 +2688,10 @@ static int run_noalloc(const pw_afd_args *a, const float *vel, const float *src,
   const size_t o_A = cv.add(nfield * 4);
   const size_t o_B = cv.add(nfield * 4);
   const size_t o_w = cv.add((size_t)p.nb * 4);
-  const int nzt = (int)round_up(g.nz, 4);  // the z table is read four at a time
-  const size_t o_t = cv.add((size_t)(nzt + g.nx + g.ny) * 4);
+  // the z table is read four at a time: up to three factors of the next table
+  // (or of the slice behind it) for cells beyond nz, which stay zero whatever
+  // finite factor they meet, so no padding takes a byte of the fixed array
+  const size_t o_t = cv.add((size_t)(g.nz + g.nx + g.ny) * 4);
   const size_t o_rec = cv.add(dat ? (size_t)nt * nrec * 4 : 0);
   const size_t o_mx = cv.add(16);
   const size_t need = cv.total();
@@ -2720,7 +2722,7 @@ static int run_noalloc(const pw_afd_args *a, const float *vel, const float *src,
   float *vv = at<float>(base, o_vv);
   float *A = at<float>(base, o_A), *B = at<float>(base, o_B);
   float *d_w = at<float>(base, o_w);
-  float *d_wz = at<float>(base, o_t), *d_wx = d_wz + nzt, *d_wy = d_wx + g.nx;
+  float *d_wz = at<float>(base, o_t), *d_wx = d_wz + g.nz, *d_wy = d_wx + g.nx;
   float *rec = at<float>(base, o_rec);
   unsigned int *mx = at<unsigned int>(base, o_mx);
 
@@ -2766,7 +2768,7 @@ static int run_noalloc(const pw_afd_args *a, const float *vel, const float *src,
       PW_CUDA(cudaStreamSynchronize(st));
     }
   }
-  taper_table_kernel<<<ceil_div(nzt, 256), 256, 0, st>>>(d_w, p.nb, nzt, p.nz2, d_wz);
+  taper_table_kernel<<<ceil_div(g.nz, 256), 256, 0, st>>>(d_w, p.nb, g.nz, p.nz2, d_wz);
   if (two_d) {
     taper_table_kernel<<<1, 32, 0, st>>>(d_w, 0, 1, 1, d_wx);  // dummy axis: factor 1
     taper_table_kernel<<<ceil_div(g.ny, 256), 256, 0, st>>>(d_w, p.nb, g.ny, p.nx2, d_wy);
