@@ -1704,11 +1704,12 @@ static int plan_tile(bool tri, int G, int nsm, bool tma, Plan &p) {
   return PW_OK;
 }
 
-// A warp-tile variant is asked for.
+// A warp-tile variant is asked for: a tile shape, the TMA ring (PW_AFD_TMA=0
+// only declines it), or any setting of the columns per lane or the B / vv ring.
 static bool tile_selected(int G) {
   int a, b;
   tile_override(G, a, b);
-  return a > 0 || getenv("PW_AFD_TMA") || getenv("PW_AFD_SPLIT") || getenv("PW_AFD_NC");
+  return a > 0 || tile_use_tma() || getenv("PW_AFD_SPLIT") || getenv("PW_AFD_NC");
 }
 
 static int make_plan(const pw_afd_args *a, bool tri, int G, Plan &p, bool allow_tma = true) {

@@ -29,7 +29,8 @@ def _environment(monkeypatch, env):
     monkeypatch.setenv("PW_AFD_VERBOSE", "1")
 
 
-@pytest.mark.parametrize("env", [{}])
+# nothing set; the TMA ring declined, which selects nothing either
+@pytest.mark.parametrize("env", [{}, {"PW_AFD_TMA": "0"}])
 def test_default_3d_step_bit_exact_vs_reference(golden, cuda_lib, monkeypatch, capfd, env):
     """80 x 72 x 64 interior, nbt 10, nt 60: the traces and snapshots of 2
     sources, and the snapshots of the time reversal of one x-band's traces,
