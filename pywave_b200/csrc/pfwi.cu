@@ -48,9 +48,11 @@ enum Mode { FWD = 0, ADJ_REF = 1, ADJ_EXACT = 2 };
 // Below xmin (the tiny values at the edge of a wavefield) and above xmax, or
 // when the check fails: div_f64; for NaN or infinity, or a divisor that is not
 // finite and positive (the square of a spacing over- or underflows): __fdiv_rn.
+// div_f64 is checked against __fdiv_rn as well (div_f64_check_kernel); a
+// divisor that failed would take __fdiv_rn there.
 struct DivC {
   float d, zh, zl, xmin, xmax;  // xmin > xmax: no numerator takes the method
-  int f64;                      // 1: d is finite and positive, div_f64 applies
+  int f64;                      // 1: d is finite and positive and passed the check of div_f64
   double dd, rd;                // d and RN(1/d)
 };
 
@@ -816,6 +818,23 @@ __global__ void fastdiv_check_kernel(float d, float zh, float zl, float scale) {
   if (__float_as_uint(q) != __float_as_uint(__fdiv_rn(x, d))) atomicAdd(&fastdiv_bad, 1u);
 }
 
+// div_f64 against __fdiv_rn, both signs: for the 2^23 significands of x in
+// [scale, 2 scale), where the quotient is a normal float (so for every x of
+// such a quotient: no intermediate value of div_f64 leaves double's normal
+// range, and scaling x by 2^k scales each step exactly), and for every x with
+// bits up to `tiny`, which include all whose quotient is subnormal.
+__global__ void __launch_bounds__(256) div_f64_check_kernel(DivC c, float scale, unsigned int tiny) {
+  const unsigned int n = (1u << 23) + tiny, stride = gridDim.x * 256;
+  unsigned int bad = 0;
+  for (unsigned int i = blockIdx.x * 256 + threadIdx.x; i < n; i += stride) {
+    const float x = i < (1u << 23) ? __fmul_rn(scale, __uint_as_float(0x3f800000u | i))
+                                   : __uint_as_float(i - (1u << 23) + 1u);
+    bad += __float_as_uint(div_f64(x, c.dd, c.rd)) != __float_as_uint(__fdiv_rn(x, c.d));
+    bad += __float_as_uint(div_f64(-x, c.dd, c.rd)) != __float_as_uint(__fdiv_rn(-x, c.d));
+  }
+  if (bad) atomicAdd(&fastdiv_bad, bad);
+}
+
 // DivC for d (cached per process: the result depends on d only).
 static int prepare_div(float d, DivC &c) {
   static std::mutex mu;
@@ -871,10 +890,20 @@ static int prepare_div(float d, DivC &c) {
         c.xmax = (float)hi;
       }
     }
+    // quotients below FLT_MIN have numerators below FLT_MIN d (a margin of two)
+    const float top = (float)std::min(2. * FLT_MIN * d + 2. * FLT_TRUE_MIN, (double)FLT_MAX);
+    unsigned int tiny, bad = 0;
+    memcpy(&tiny, &top, 4);
+    const float scale = std::max(std::ldexp(1.f, (int)std::floor(std::log2((double)d))), FLT_MIN);
+    PW_CUDA(cudaMemcpyToSymbol(fastdiv_bad, &bad, sizeof bad));
+    div_f64_check_kernel<<<8 * 148, 256>>>(c, scale, tiny);
+    PW_CUDA(cudaGetLastError());
+    PW_CUDA(cudaMemcpyFromSymbol(&bad, fastdiv_bad, sizeof bad));
+    c.f64 = bad == 0;
   }
   if (getenv("PW_PFWI_VERBOSE"))
-    fprintf(stderr, "pfwi: division by %.9g: zh %.9g zl %.9g range [%.3g, %.3g]\n", d, c.zh, c.zl,
-            c.xmin, c.xmax);
+    fprintf(stderr, "pfwi: division by %.9g: zh %.9g zl %.9g range [%.3g, %.3g], FP64 %d\n", d,
+            c.zh, c.zl, c.xmin, c.xmax, c.f64);
   cache[key] = c;
   return PW_OK;
 }
