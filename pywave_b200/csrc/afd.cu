@@ -92,8 +92,8 @@ struct StepArgs {
   int nbz, nbx, nby, nz1, nx1, ny1;  // interior = [nb, nb+n1) per kernel axis
   float *wfd;                  // this step's snapshot [ny1][nx1][nz1] (group 0) or null
   float *img;                  // image accumulator (field layout) or null
-  // warp-plane counts of the 3-D step paths, or null (warp-tile kernels
-  // only): [0..3] TRI paths 0..3, [4..7] forward paths 0..3
+  // 3-D counters of the verbose print, or null: [0..3] TRI, [4..7] forward.
+  // Warp-tile kernels: warp-planes by the path taken; quad3_kernel: see quad_stats
   unsigned long long *stats;
   int *err;  // set to nonzero by a warp-tile kernel whose bounded wait gave up
 };
@@ -344,10 +344,12 @@ __device__ __forceinline__ int quad_slot(const StepArgs &a, unsigned block, int 
   return (int)item - group * a.nq.d + 1;
 }
 
-// Counts of the warps' groups by taper class, kept only when a.stats is set
-// (one warp-plane each): 0 no taper and no mask, 1 y taper only, 2 z / x taper
-// only, 3 anything else (both, masks, sources, injection).  [0..3] TRI,
-// [4..7] forward.
+// What the warps of a step meet, counted only when a.stats is set (one per
+// group and step): 0 no taper and no mask, 1 y taper only, 2 z / x taper only,
+// 3 anything else (both, masks, sources, injection).  The step runs the same
+// code whatever the class: the counts describe the grid.  They stay in the step
+// because a kernel of their own left it 4% slower forward (261^3; 68 registers
+// in place of 64, 7 CTAs per SM in place of 8).
 template <bool TRI>
 __device__ __forceinline__ void quad_stats(const StepArgs &a, bool live, int slot, int ix, int y) {
   const Geo &g = a.g;
@@ -399,7 +401,8 @@ __global__ void __launch_bounds__(32 * QXW, 6)
 // 2-D: QW2 columns of the kernel's y (the model's x) per CTA, and one warp per
 // column and group (a 2-D step is a chain of load latencies: the groups in
 // turn in one thread took 4.8 us per step of 261^2 and 4 groups, in warps of
-// their own 3.0, with the fixed operands read early 2.4).  The image product meets the groups in shared memory.
+// their own 3.0, with the fixed operands read early 2.4).  The image product
+// meets the groups in shared memory.
 template <bool TRI, bool SNAP, bool EARLY>
 __global__ void __launch_bounds__(32 * QW2 * (TRI ? MAXG : 1))
     quad2_kernel(const __grid_constant__ StepArgs a) {
@@ -1547,8 +1550,8 @@ static void plan_quad(bool tri, int G, Plan &p) {
   p.fn = tri ? quad_fn<true, false>(two_d, early) : quad_fn<false, false>(two_d, early);
   p.fn_snap = tri ? quad_fn<true, true>(two_d, early) : quad_fn<false, true>(two_d, early);
   if (getenv("PW_AFD_VERBOSE"))
-    fprintf(stderr, "afd quad plan: G=%d nq=%d threads=%d grid=%ux%u\n", G, p.nq.d, p.threads,
-            p.grid.x, p.grid.y);
+    fprintf(stderr, "afd quad plan: G=%d nq=%d threads=%d grid=%ux%ux%u early=%d\n", G, p.nq.d,
+            p.threads, p.grid.x, p.grid.y, p.grid.z, early);
 }
 
 // Tile override for measurements: PW_AFD_TILE_G<G>="a,b" fixes the first two
@@ -2094,7 +2097,8 @@ static int run(const pw_afd_args *a, int G, const int *group, const float *vel, 
   const size_t o_gid = cv.add(use_gid ? nrec * 4 : 0);
   const size_t o_wfd = cv.add(wfd && host ? (size_t)ntsnap * nvel * 4 : 0);
   const size_t o_mx = cv.add(16);
-  // PW_AFD_VERBOSE: also count which paths the 3-D step kernels took
+  // PW_AFD_VERBOSE: also count the paths of the warp-tile kernels, or what the
+  // quad kernel's warps meet
   const bool want_stats = !two_d && getenv("PW_AFD_VERBOSE") != nullptr;
   const size_t o_stats = cv.add(want_stats ? 8 * sizeof(unsigned long long) : 0);
   const size_t o_err = cv.add(p.tma ? 16 : 0);
@@ -2319,6 +2323,11 @@ static int run(const pw_afd_args *a, int G, const int *group, const float *vel, 
   if (want_stats) {
     unsigned long long c[8];
     PW_CUDA(cudaMemcpy(c, s.stats, sizeof c, cudaMemcpyDeviceToHost));
+    if (p.quad) {  // one code path: say what the counts are before they are listed
+      const unsigned long long *k = c + (tri ? 0 : 4), per = (unsigned long long)G * nt;
+      fprintf(stderr, "afd quad warps per step: plain=%llu y_taper=%llu zx_taper=%llu other=%llu\n",
+              k[0] / per, k[1] / per, k[2] / per, k[3] / per);
+    }
     fprintf(stderr,
             "afd tile paths (warp-planes): tri_path0=%llu tri_path1=%llu tri_path2=%llu "
             "tri_path3=%llu fwd_path0=%llu fwd_path1=%llu fwd_path2=%llu fwd_path3=%llu\n",

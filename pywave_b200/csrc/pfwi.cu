@@ -991,8 +991,8 @@ static int setup(const pw_fwi_args *a, Setup &S, bool passive = false) {
   PW_CHECK(S.rz >= 4 && S.rz < S.pnz - 4, PW_ERR_SHAPE, "receiver depth in the zero border");
   if (getenv("PW_PFWI_VERBOSE")) {
     // depth class of the padded grid: columns of up to 64 or 128 float4, and
-    // how many such segments a column has (the step kernel's lanes cross
-    // columns and use neither)
+    // how many such segments a column has.  The step kernel's lanes cross
+    // columns and use neither; launch_one prints what it launches
     const int nz4 = ceil_div(S.pnz, 4), zw = nz4 <= 64 ? 64 : 128;
     fprintf(stderr, "pfwi plan: padded %d x %d, ZW=%d ztiles=%d\n", S.pnz, S.pnx, zw,
             ceil_div(nz4, zw));
@@ -1007,6 +1007,9 @@ static int launch_one(const Setup &S, PfArgs &p, int nshots, cudaStream_t st) {
   if (p.prev == MODE) {
     PW_CUDA(launch_pdl(pf_step_kernel<MODE, PAS>, grid, dim3(32 * PF_XW), 0, st, p));
   } else {
+    if (getenv("PW_PFWI_VERBOSE"))
+      fprintf(stderr, "pfwi step: mode=%d nz4=%d shots=%d grid=%ux%u threads=%d zig=%d\n", MODE,
+              p.nz4.d, nshots, grid.x, grid.y, 32 * PF_XW, p.zig);
     pf_step_kernel<MODE, PAS><<<grid, 32 * PF_XW, 0, st>>>(p);
     PW_CUDA(cudaGetLastError());
   }
