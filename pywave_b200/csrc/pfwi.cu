@@ -47,7 +47,8 @@ enum Mode { FWD = 0, ADJ_REF = 1, ADJ_EXACT = 2 };
 // intermediate values stay normal, which |x| in [xmin, xmax] ensures.
 // Below xmin (the tiny values at the edge of a wavefield) and above xmax, or
 // when the check fails: div_f64; for NaN or infinity, or a divisor that is not
-// finite and positive (the square of a spacing over- or underflows): __fdiv_rn.
+// finite and positive (the square of a spacing over- or underflows): __fdiv_rn,
+// in step kernels of their own.
 // div_f64 is checked against __fdiv_rn as well (div_f64_check_kernel); a
 // divisor that failed would take __fdiv_rn there.
 struct DivC {
@@ -138,9 +139,11 @@ __device__ __forceinline__ float div_f64(float v, double d, double rd) {
 // method, two values per op.  All zero (ahead of the numerical wavefront):
 // zero.  Otherwise (the shell of tiny values around that zone, which crosses
 // most columns while a wave expands) through FP64, or by __fdiv_rn where a
-// numerator is infinite or NaN or a divisor is not finite and positive (x / inf
-// is 0 and 0 / 0 NaN, which the other forms do not give).  The first test is 8
-// three-operand minima and maxima for the 8 numerators.
+// numerator is infinite or NaN.  The first test is 8 three-operand minima and
+// maxima for the 8 numerators.  IEEE: __fdiv_rn for every numerator, where a
+// divisor is not finite and positive (x / inf is 0 and 0 / 0 NaN, which the
+// other forms do not give); as a test in the common kernel it cost the exact
+// gradient 0.6% (16 shots of 420 x 720, 20.44 -> 20.56 us per step).
 // The sign of a zero quotient is not kept (these forms can give +0 for -0):
 // no output depends on it.  The sum of the quotients is then +0 where it
 // should be -0 only if both numerators are -0, for which the centre value c
@@ -148,10 +151,19 @@ __device__ __forceinline__ float div_f64(float v, double d, double rd) {
 // becomes -0); the update (2c - b) + V t has 2c - b = +0 - b, which is not
 // -0, so adding +0 or -0 gives the same bits, and the gradient sums start at
 // +0, which adding either zero leaves unchanged.
+template <bool IEEE>
 __device__ __forceinline__ void div4_sum(const f2 (&tx)[2], const f2 (&tz)[2], const DivC &cx,
                                          const DivC &cz, float xlo, float xhi, bool unused,
                                          f2 (&t)[2]) {
   const float4 x = join2(tx[0], tx[1]), z = join2(tz[0], tz[1]);
+  float4 r;
+  if (IEEE) {
+#pragma unroll 1
+    for (int e = 0; e < 4; e++) set_el(r, e, fadd(__fdiv_rn(el(x, e), cx.d), __fdiv_rn(el(z, e), cz.d)));
+    t[0] = lo2(r);
+    t[1] = hi2(r);
+    return;
+  }
   const float mx = max3abs(max3abs(max3abs(x.x, x.y, x.z), x.w, z.x), z.y, max3abs(z.z, z.w, 0.f));
   const float mn = min3abs(min3abs(min3abs(x.x, x.y, x.z), x.w, z.x), z.y, min3abs(z.z, z.w, z.w));
   const f2 xh = pk2(cx.zh, cx.zh), xl = pk2(cx.zl, cx.zl);
@@ -162,11 +174,9 @@ __device__ __forceinline__ void div4_sum(const f2 (&tx)[2], const f2 (&tz)[2], c
       t[h] = add2(fma2(tx[h], xh, mul2(tx[h], xl)), fma2(tz[h], zh, mul2(tz[h], zl)));
     return;
   }
-  const bool f64 = cx.f64 && cz.f64;
   t[0] = t[1] = 0ull;
-  if (f64 && mx == 0.f) return;
-  float4 r;
-  if (f64 && mx <= FLT_MAX) {
+  if (mx == 0.f) return;
+  if (mx <= FLT_MAX) {
 #pragma unroll
     for (int e = 0; e < 4; e++)
       set_el(r, e, fadd(div_f64(el(x, e), cx.dd, cx.rd), div_f64(el(z, e), cz.dd, cz.rd)));
@@ -203,7 +213,7 @@ __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast
 // all that no step of the mode writes read (and the imaging's division done)
 // before the previous step has ended, forward and reference adjoint take 3.4
 // us on average, 3.9 with all reads after it.
-template <int MODE, bool PAS>
+template <int MODE, bool PAS, bool IEEE>
 __global__ void __launch_bounds__(32 * PF_XW, MODE == ADJ_REF || PAS ? 5 : 6)
     pf_step_kernel(const __grid_constant__ PfArgs a) {
   const int s = zigzag(a.it & a.zig, blockIdx.y, gridDim.y);
@@ -337,7 +347,7 @@ __global__ void __launch_bounds__(32 * PF_XW, MODE == ADJ_REF || PAS ? 5 : 6)
       tx2[h] = tx;
       tz2[h] = tz;
     }
-    div4_sum(tx2, tz2, a.divx, a.divz, a.xlo, a.xhi, !(lz_any && lx_ok), t2);
+    div4_sum<IEEE>(tx2, tz2, a.divx, a.divz, a.xlo, a.xhi, !(lz_any && lx_ok), t2);
   }
   float4 term4 = join2(t2[0], t2[1]);
   if (!(lz_full && lx_ok)) {
@@ -1004,13 +1014,15 @@ template <int MODE, bool PAS = false>
 static int launch_one(const Setup &S, PfArgs &p, int nshots, cudaStream_t st) {
   const long long lanes = (long long)p.nz4.d * ceil_div(S.pnx, PF_XW);
   const dim3 grid((unsigned)ceil_div(lanes, 32), (unsigned)nshots);
+  auto fn = S.divx.f64 && S.divz.f64 ? pf_step_kernel<MODE, PAS, false>
+                                     : pf_step_kernel<MODE, PAS, true>;
   if (p.prev == MODE) {
-    PW_CUDA(launch_pdl(pf_step_kernel<MODE, PAS>, grid, dim3(32 * PF_XW), 0, st, p));
+    PW_CUDA(launch_pdl(fn, grid, dim3(32 * PF_XW), 0, st, p));
   } else {
     if (getenv("PW_PFWI_VERBOSE"))
       fprintf(stderr, "pfwi step: mode=%d nz4=%d shots=%d grid=%ux%u threads=%d zig=%d\n", MODE,
               p.nz4.d, nshots, grid.x, grid.y, 32 * PF_XW, p.zig);
-    pf_step_kernel<MODE, PAS><<<grid, 32 * PF_XW, 0, st>>>(p);
+    fn<<<grid, 32 * PF_XW, 0, st>>>(p);
     PW_CUDA(cudaGetLastError());
   }
   p.prev = MODE;
