@@ -18,8 +18,11 @@
 // resident_kernel (every step in one launch); the other 2-D runs and all 3-D
 // runs take the quad kernels, one float4 of z cells per thread and step.  The
 // warp-tile kernels, which march 3-D patches along y through shared-memory
-// rings, are kept as selectable variants (PW_AFD_TMA, PW_AFD_SPLIT, PW_AFD_NC,
-// PW_AFD_TILE_G<G>); their TRI images are formed by image_kernel.
+// rings, run only where a switch selects them (PW_AFD_TMA=1, PW_AFD_SPLIT,
+// PW_AFD_NC, PW_AFD_TILE_G<G>).  They are slower (217-305 against 215 us per
+// 261^3 step of 4 groups) and serve as second implementations of the 3-D step,
+// by per-lane copies and by TMA, that the tests hold against the same
+// reference digests.  Their TRI images are formed by image_kernel.
 //
 // Two buffers per wavefield: at step k the kernel reads A = u_k and B =
 // u_{k-1} (as stored, tapered once) and overwrites B with u_{k+1}.  The
@@ -192,11 +195,13 @@ __device__ __forceinline__ float4 taper_quad(const float4 &v, const float (&wz)[
 // an imaging step is formed in registers.  No march, no shared memory, no
 // barrier: neighbours come from L1 and L2, and many small independent threads
 // hide the latency.  Same float evaluation order as the reference.
-// Bound: 261^3 time reversal of 4 groups, L2 to L1 traffic (2.3 GB per step
-// at 215 us; without any neighbour load it takes 180, the 925 MB of fields at
-// the measured copy rate 143); 261^3 forward 56 us (56 without neighbour
-// loads); 141^3 and the 2-D sections, which stay in L2, launch and load
-// latency.  Measured per step against the kernels before (warp patches that
+// Bound: 261^3 time reversal of 4 groups, load latency and L1's data pipe
+// (215 us; without any neighbour load 180, the 925 MB of fields at the
+// measured copy rate 143; three quarters of the stall cycles wait for loads,
+// L1's load pipe is 78% busy, DRAM 0.73 of the copy rate, issue 44%; the 2.3 GB
+// from L2 take 31% of what L2 can return); 261^3 forward 56 us (56 without
+// neighbour loads); 141^3 and the 2-D sections, which stay in L2, launch and
+// load latency.  Measured per step against the kernels before (warp patches that
 // march y through shared-memory rings; 2-D columns marched through a
 // per-thread ring): 261^3, 4 groups 231 -> 215 us (183 instructions per
 // float4 instead of 263); 261^3 forward 103 -> 56; 141^3 forward 25 -> 9.6;
@@ -205,7 +210,7 @@ __device__ __forceinline__ float4 taper_quad(const float4 &v, const float (&wz)[
 // the 3-D grids; CTAs of 4 x 4 columns 250 / 84 / 12.8, of 8 slots x 4 x 4
 // 226 / 67 / 10.9; the groups of a launch in separate CTAs 242.
 constexpr int QXW = 4;  // 3-D: columns (warps) per CTA, of one plane
-constexpr int QW2 = 4;           // 2-D: columns (warps) per CTA
+constexpr int QW2 = 4;  // 2-D: columns (warps) per CTA
 
 __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 

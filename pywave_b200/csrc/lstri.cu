@@ -83,10 +83,6 @@ __device__ __forceinline__ void qset(float4 &v, int e, float x) {
   else if (e == 2) v.z = x;
   else v.w = x;
 }
-// cell j (-4..7) of the z window made of the quads below, at and above
-__device__ __forceinline__ float zwin(const float4 &lo, const float4 &c, const float4 &hi, int j) {
-  return j < 0 ? qel(lo, j + 4) : (j < 4 ? qel(c, j) : qel(hi, j - 4));
-}
 
 // Static description of one quad (column ix, quad k): bit 0 live (has a
 // stencil cell), bits 1-4 stencil cell e, bits 5-8 interior (source /
@@ -544,11 +540,12 @@ static int check_args(const pw_fwi_args *a, bool need_shots) {
 // quads in brackets: one shot [2500] 1.2 / 2.1, [6400] 1.6 / 2.1, [8100]
 // 2.0 / 2.2, [12100] 2.3 / 2.1, [28600] 3.8 / 2.1; adjoint [6400] 1.8 / 2.1,
 // [8100] 2.4 / 2.1, [28600] 5.1 / 2.1; 8 shots, two waves [1600] 1.9 / 2.1,
-// [2500] 2.4 / 2.0, [28600] 7.9 / 4.3.  Several shots that fit in one wave
-// stay one launch at every size, although steps are faster from 10000 quads
-// on ([28600], 2 shots: 3.9 / 2.3): the host thread is free meanwhile.  So do
-// shots whose fields would take more than 256 MB of workspace (or a grid of
-// more than 65535 rows), which the resident form does without.
+// [2500] 2.4 / 2.0, [28600] 7.9 / 4.3.  The rule is not applied to several
+// shots that fit in one wave: they are one resident launch at every size, as
+// the suite expects of them by default, although steps are faster from 10000
+// quads on ([28600], 2 shots: 3.9 / 2.3; PW_LSTRI_RESIDENT=0 takes them).  Shots
+// whose fields would take more than 256 MB of workspace (or a grid of more
+// than 65535 rows) stay resident too, which does without.
 // PW_LSTRI_RESIDENT=1 keeps every operator resident where it fits, 0 none.
 static void make_plan(const pw_fwi_args *a, bool adj, int nshots, Plan &p) {
   p.nzp = a->nz + 2 * a->nb;

@@ -2248,7 +2248,8 @@ __host__ __device__ inline long long off3(const Args &a, int iz, int ix, int iy)
 // two z neighbours, the previous field and V; for the adjoint the forward term
 // and the gradient), as the 2-D step does.  Shots are the fastest block index,
 // so the shots of a cell share V through L2.
-// Bound: L2 to L1 traffic and load latency (21 float4 loads per float4; DRAM
+// Bound: load latency and L1's data pipe (21 float4 loads per float4; L1's load
+// pipe is 75% busy, issue 55%, the return from L2 31%; DRAM
 // would allow 57 us forward and 80 us adjoint).  Measured, one launch, 2 shots
 // of 160 x 240 x 240, average of forward and adjoint: 95.6 us (157 with the
 // former 3-plane shared-memory ring and a barrier per plane); 1 shot of 200 x

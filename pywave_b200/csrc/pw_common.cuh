@@ -191,9 +191,9 @@ __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.laun
 __device__ __forceinline__ int zigzag(int it, int b, int n) { return (it & 1) ? n - 1 - b : b; }
 // 1 where a launch's fields of `bytes` leave L2 between steps: above half of
 // its 126 MB, since lines read by both dies are held twice.  Measured per
-// step, with / without: 98 MB (12 uneven 2-D shots) 29.1 / 33.6 us (27.4 now), 83 MB (32
-// shots of 420 x 720, gradient) 42.9 / 46.0, 213 MB (261^3) 55.8 / 57.3; below,
-// where all stays in L2, 41 MB (16 shots) 20.7 / 20.2, 15 MB 6.7 / 6.4.
+// step, with / without: 98 MB (12 uneven 2-D shots) 27.9 / 31.9 us, 83 MB (32
+// shots of 420 x 720, gradient) 42.7 / 47.1, 213 MB (261^3) 56.3 / 58.3; below,
+// where all stays in L2, 41 MB (16 shots) 20.3 / 20.5, 15 MB 6.5 / 6.4.
 inline int zigzag_pays(size_t bytes) { return bytes > (size_t(60) << 20) ? 1 : 0; }
 
 // Packed pairs of floats for sm_100's f32x2 pipe: add / sub / mul.rn.f32x2
