@@ -266,8 +266,19 @@ def job_rate(units_per_rank_step, steps, world, ms_max):
     return units_per_rank_step * steps * world / (ms_max / 1e3)
 
 
+def reference_built():
+    """Whether the reference's own afdcfun extension is there to be imported."""
+    from importlib.machinery import PathFinder
+    return PathFinder.find_spec("afdcfun", [os.path.join(ROOT, "oracle", "_ref")]) is not None
+
+
 def run_reference(args, rank):
     if rank != 0:
+        return
+    if not reference_built():
+        print(json.dumps({"impl": "reference", "unavailable":
+                          "afdcfun is not built under oracle/_ref (`make -C oracle ref` needs the "
+                          "pywave sources)"}), flush=True)
         return
     n = args.n
     workers = max(1, min(os.cpu_count() or 1, 16))
