@@ -114,7 +114,13 @@ __device__ __forceinline__ unsigned quad_flags(const Args &a, int ix, int k) {
 // first, and 2 A is formed as A + A.  Cells outside the stencil stay zero.
 // inj: modelling, the source samples of the interior cells (mod[it]); adjoint,
 // element 0 the data sample of the data row.
-template <bool ADJ>
+// PRED: the source samples and the cells outside the stencil are chosen per
+// cell without a branch around them.  Faster where a step is one cluster
+// barrier and has few quads per thread, and only in modelling: resident, 20 x
+// 30 with 10 sponge cells, us per step with branches / without: modelling 0.96
+// / 0.93 (8 shots 1.88 / 1.83), 60 x 100 with 30 1.45 / 1.43, adjoints 0.95 /
+// 0.97 and 1.55 / 1.62.
+template <bool ADJ, bool PRED>
 __device__ __forceinline__ float4 quad_step(const Args &a, unsigned f, const float4 (&sx9)[9],
                                             const float4 &szl, const float4 &szh, const float4 &A,
                                             const float4 &V, const float4 &B, const float4 &wz4,
@@ -150,7 +156,7 @@ __device__ __forceinline__ float4 quad_step(const Args &a, unsigned f, const flo
   }
   float4 n = join2(n2[0], n2[1]);
   if (!ADJ) {
-    if (f & (0xFu << 5)) {
+    if (PRED || (f & (0xFu << 5))) {
 #pragma unroll
       for (int e = 0; e < 4; e++)
         if (f & (32u << e)) qset(n, e, fadd(qel(n, e), fmul(qel(inj, e), qel(V, e))));
@@ -161,7 +167,7 @@ __device__ __forceinline__ float4 quad_step(const Args &a, unsigned f, const flo
       if (e == a.depth - 4 * k) qset(n, e, fadd(qel(n, e), inj.x));
   }
   float4 r = join2(mul2(mul2(lo2(n), lo2(wz4)), wx2), mul2(mul2(hi2(n), hi2(wz4)), wx2));
-  if ((f & 0x1Eu) != 0x1Eu) {
+  if (PRED || (f & 0x1Eu) != 0x1Eu) {
 #pragma unroll
     for (int e = 0; e < 4; e++)
       if (!(f & (2u << e))) qset(r, e, 0.f);
@@ -294,7 +300,8 @@ __global__ void __launch_bounds__(RNTH) resident_kernel(const __grid_constant__ 
         szh = quad_mul(a.one, szh, Vs[o + 1]);
       }
       quad_out<ADJ>(a, mod, dat, f, ADJ ? sx9[4] : A, ix, k, it);
-      const float4 r = quad_step<ADJ>(a, f, sx9, szl, szh, A, V, nxt[o], wzs[k], wxs[c], inj[j], k);
+      const float4 r =
+          quad_step<ADJ, !ADJ>(a, f, sx9, szl, szh, A, V, nxt[o], wzs[k], wxs[c], inj[j], k);
       inj[j] = load_inj<ADJ>(a, mod, dat, f, ix, k, ADJ ? it - 1 : it + 1);
       nxt[o] = r;
       if (f & (1u << 10)) *cl_map(nxt + o + w * nq, rank - 1) = r;
@@ -345,7 +352,7 @@ __global__ void __launch_bounds__(SNTH) step_kernel(const __grid_constant__ Args
     asm volatile("prefetch.global.L2 [%0];" ::"l"(next + e));
   }
   quad_out<ADJ>(a, mod, dat, f, sx9[4], ix, k, a.it);
-  const float4 r = quad_step<ADJ>(a, f, sx9, szl, szh, A, V, B, wz, wx, inj, k);
+  const float4 r = quad_step<ADJ, false>(a, f, sx9, szl, szh, A, V, B, wz, wx, inj, k);
   a.Y[o] = r;
   if (ADJ) a.Wn[o] = quad_mul(a.one, r, V);
 }
