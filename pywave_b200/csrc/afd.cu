@@ -19,8 +19,9 @@
 // runs take the quad kernels, one float4 of z cells per thread and step.  The
 // warp-tile kernels, which march 3-D patches along y through shared-memory
 // rings, run only where a switch selects them (PW_AFD_TMA=1, PW_AFD_SPLIT,
-// PW_AFD_NC, PW_AFD_TILE_G<G>).  They are slower (217-305 against 215 us per
-// 261^3 step of 4 groups) and serve as second implementations of the 3-D step,
+// PW_AFD_NC, PW_AFD_TILE_G<G>).  They are slower (217-305 against 213 us per
+// 261^3 step of 4 groups; level with it for 2 groups on the largest grids, see
+// quad3_tri_fn) and serve as second implementations of the 3-D step,
 // by per-lane copies and by TMA, that the tests hold against the same
 // reference digests.  Their TRI images are formed by image_kernel.
 //
@@ -196,14 +197,14 @@ __device__ __forceinline__ float4 taper_quad(const float4 &v, const float (&wz)[
 // barrier: neighbours come from L1 and L2, and many small independent threads
 // hide the latency.  Same float evaluation order as the reference.
 // Bound: 261^3 time reversal of 4 groups, load latency and L1's data pipe
-// (215 us; without any neighbour load 180, the 925 MB of fields at the
+// (213 us; without any neighbour load 180, the 925 MB of fields at the
 // measured copy rate 143; three quarters of the stall cycles wait for loads,
-// L1's load pipe is 78% busy, DRAM 0.73 of the copy rate, issue 44%; the 2.3 GB
-// from L2 take 31% of what L2 can return); 261^3 forward 56 us (56 without
+// L1's load pipe is 78% busy, DRAM 0.73 of the copy rate, issue 43%; the 2.3 GB
+// from L2 take 30% of what L2 can return); 261^3 forward 56 us (56 without
 // neighbour loads); 141^3 and the 2-D sections, which stay in L2, launch and
 // load latency.  Measured per step against the kernels before (warp patches that
 // march y through shared-memory rings; 2-D columns marched through a
-// per-thread ring): 261^3, 4 groups 231 -> 215 us (183 instructions per
+// per-thread ring): 261^3, 4 groups 231 -> 213 us (183 instructions per
 // float4 instead of 263); 261^3 forward 103 -> 56; 141^3 forward 25 -> 9.6;
 // 561 x 1561 forward 8.2 -> 3.6; 12 uneven shots 44.7 -> 27.4.  Marching up to 8
 // planes per thread with the y neighbours in registers: 217 / 77 / 13 us on
@@ -224,7 +225,8 @@ __device__ __forceinline__ void square_into(float4 &prod, const float4 &u) {
 // Groups [g0, g1) of one float4; the square product of their new values in
 // group order multiplies `prod` (imaging steps).  EARLY: what no step writes
 // is read before the previous step has ended (else the kernel waits first).
-template <bool XT, bool TRI, bool SNAP, bool EARLY>
+// UN: how many groups the loop is unrolled by.
+template <bool XT, bool TRI, bool SNAP, bool EARLY, int UN = 1>
 __device__ __forceinline__ void quad_update(const StepArgs &a, int slot, int ix, int y, int it,
                                             bool swap, int g0, int g1, float4 &prod,
                                             float4 *last = nullptr) {
@@ -262,7 +264,7 @@ __device__ __forceinline__ void quad_update(const StepArgs &a, int slot, int ix,
     pdl_wait();
     pdl_launch();
   }
-#pragma unroll 1
+#pragma unroll UN
   for (int gi = TRI ? g0 : 0; gi < (TRI ? g1 : 1); gi++) {
     const float *A = (swap ? a.nxt[gi] : a.cur[gi]) + o;
     float *B = (swap ? const_cast<float *>(a.cur[gi]) : a.nxt[gi]) + o;
@@ -382,8 +384,9 @@ __device__ __forceinline__ void quad_stats(const StepArgs &a, bool live, int slo
   }
 }
 
-// 3-D: QXW columns of one plane per CTA
-template <bool TRI, bool SNAP, bool EARLY>
+// 3-D: QXW columns of one plane per CTA.  NG: the groups of a time reversal, known
+// at compile time (0: a.ngroups of them, the loop not unrolled), see quad3_tri_fn
+template <bool TRI, bool SNAP, bool EARLY, int NG = 0>
 __global__ void __launch_bounds__(32 * QXW, 6)
     quad3_kernel(const __grid_constant__ StepArgs a) {
   int group;
@@ -399,7 +402,8 @@ __global__ void __launch_bounds__(32 * QXW, 6)
   if (a.stats != nullptr) quad_stats<TRI>(a, live, slot, ix, y);
   if (!live) return;
   float4 prod = make_float4(1.f, 1.f, 1.f, 1.f);
-  quad_update<true, TRI, SNAP, EARLY>(a, slot, ix, y, a.it, false, 0, a.ngroups, prod);
+  quad_update<true, TRI, SNAP, EARLY, NG ? NG : 1>(a, slot, ix, y, a.it, false, 0,
+                                                   NG ? NG : a.ngroups, prod);
   if (SNAP && TRI) quad_image(a, slot, ix, y, prod);
 }
 
@@ -1536,10 +1540,31 @@ struct Plan {
 // ones of up to 800 x 1700 28.8 / 27.4.
 constexpr long long EARLY_THREADS = 160000;
 
+// 3-D time reversal of one to four groups has a kernel per count: unrolled, a
+// group's loads can be issued together with vv and the tapers, which a loop
+// over the groups reads before its first pass.  Measured, us per step on average with an
+// image every 4 steps, count at run time / compile time (in brackets the
+// warp-tile kernel, which the former was behind for few groups on large grids):
+// 321^3, 1 group 155 / 129 (141), 2 groups 235 / 217 (218), 3 315 / 286 (313),
+// 4 396 / 388 (402); 461 x 321 x 221 150 / 122 (133), 227 / 209 (209), 305 / 277
+// (303), 382 / 374 (385); 221^3 51 / 44 (66), 79 / 73 (93), 106 / 97 (123),
+// 134 / 130 (149); 141^3 12.6 / 11.5, 19.8 / 18.8, 28.7 / 26.7, 37.3 / 36.3.
+template <bool SNAP, bool EARLY>
+static void *quad3_tri_fn(int G) {
+  switch (G) {
+    case 1: return (void *)quad3_kernel<true, SNAP, EARLY, 1>;
+    case 2: return (void *)quad3_kernel<true, SNAP, EARLY, 2>;
+    case 3: return (void *)quad3_kernel<true, SNAP, EARLY, 3>;
+    case 4: return (void *)quad3_kernel<true, SNAP, EARLY, 4>;
+    default: return (void *)quad3_kernel<true, SNAP, EARLY>;
+  }
+}
+
 template <bool TRI, bool SNAP>
-static void *quad_fn(bool two_d, bool early) {
+static void *quad_fn(bool two_d, bool early, int G) {
   if (two_d) return early ? (void *)quad2_kernel<TRI, SNAP, true> : (void *)quad2_kernel<TRI, SNAP, false>;
-  return early ? (void *)quad3_kernel<TRI, SNAP, true> : (void *)quad3_kernel<TRI, SNAP, false>;
+  if constexpr (TRI) return early ? quad3_tri_fn<SNAP, true>(G) : quad3_tri_fn<SNAP, false>(G);
+  else return early ? (void *)quad3_kernel<false, SNAP, true> : (void *)quad3_kernel<false, SNAP, false>;
 }
 
 static void plan_quad(bool tri, int G, Plan &p) {
@@ -1552,8 +1577,8 @@ static void plan_quad(bool tri, int G, Plan &p) {
   p.threads = 32 * (two_d ? QW2 * (tri ? G : 1) : QXW);
   p.smem = 0;
   const bool early = (long long)p.grid.x * p.grid.y * p.grid.z * p.threads <= EARLY_THREADS;
-  p.fn = tri ? quad_fn<true, false>(two_d, early) : quad_fn<false, false>(two_d, early);
-  p.fn_snap = tri ? quad_fn<true, true>(two_d, early) : quad_fn<false, true>(two_d, early);
+  p.fn = tri ? quad_fn<true, false>(two_d, early, G) : quad_fn<false, false>(two_d, early, G);
+  p.fn_snap = tri ? quad_fn<true, true>(two_d, early, G) : quad_fn<false, true>(two_d, early, G);
   if (getenv("PW_AFD_VERBOSE"))
     fprintf(stderr, "afd quad plan: G=%d nq=%d threads=%d grid=%ux%ux%u early=%d\n", G, p.nq.d,
             p.threads, p.grid.x, p.grid.y, p.grid.z, early);
